@@ -155,9 +155,9 @@ pf_status pf_sigma_download(pf_sigma_ctx* ctx, uint32_t* lits, uint64_t* offsets
  * whose solver never assigns them), then the witness stack is walked from its end:
  * a record whose other literals are all false sets its witness true. Single formula:
  * values[0 .. num_vars] (index 0 unused); its records form one dependent chain,
- * walked by one device thread. Formula batch: formula after formula, num_vars[f] + 1
+ * walked by one warp. Formula batch: formula after formula, num_vars[f] + 1
  * entries each (the first unused; the layout of pf_sigma_batch_download's eliminated
- * flags), every formula walked by its own thread, side by side. For the batched
+ * flags), every formula walked by its own warp, side by side. For the batched
  * SAT answers of many formulas; one large formula is faster on a host core. */
 pf_status pf_sigma_extend(pf_sigma_ctx* ctx, uint8_t* values);
 

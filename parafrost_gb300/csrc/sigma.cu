@@ -207,7 +207,7 @@ struct FRecFid {
         key[r] = f;
         val[r] = r;
         words[r] = en - st;
-        atom_add64(&f_words[f], (u64)(en - st));
+        if (f_words) atom_add64(&f_words[f], (u64)(en - st));
     }
 };
 struct FRecSize {
@@ -228,13 +228,15 @@ struct FRecGather {
         o[n - 1] = c.resolved[st + n - 1];
     }
 };
-// Model extension: records per formula, and the walks.
-struct FRecCount {
-    Ctx c; const u32* rstart; u32* f_recs;
-    HD void operator()(u32 r) const { atom_add(&f_recs[c.var_fid[ABS(c.resolved[rstart[r]])]], 1u); }
+// Model extension: first record per formula, and the walks.
+struct FExtendFirst {
+    const u32* fid; u32 nrec; u32* f_first;
+    HD void operator()(u32 f) const { k_extend_first(fid, nrec, f_first, f); }
 };
+#if !SIGMA_CUDA
 struct FExtendFormula { ExtendArgs a; HD void operator()(u32 f) const { k_extend_formula(a, f); } };
 struct FExtendSingle { ExtendArgs a; HD void operator()() const { k_extend_single(a); } };
+#endif
 struct FExtendClear { Ctx c; uint8_t* value; HD void operator()(u32 v) const { k_extend_clear(c, value, v); } };
 struct FExtendUnit { Ctx c; uint8_t* value; HD void operator()(u32 i) const { k_extend_unit(c, value, i); } };
 struct FExtendIn {
@@ -1758,7 +1760,7 @@ struct pf_sigma_ctx {
     // MODEL::extend (src/cpu/model.cpp:104-138) on the device for the last round's
     // result: h_values holds the caller's model of the simplified formula(s) and
     // receives the model of the original one(s). A batch's formulas are walked side
-    // by side, one thread each.
+    // by side, one warp each.
     void extend(uint8_t* h_values) {
         DBuf<uint8_t> val, packed;
         DBuf<u64> pfirst;
@@ -1788,10 +1790,18 @@ struct pf_sigma_ctx {
         a.value = val.p;
         a.nres = nresolved;
         a.err = counters.p + 1;
-        DBuf<u32> flag, scan, rstart, key, ord, k2, v2, frec, ffirst;
-        DBuf<u64> words, fw;
+        DBuf<u32> flag, scan, rstart, key, ord, k2, v2, ffirst;
+        DBuf<u64> words;
         if (!nf) {
-            if (nresolved) rt.one(FExtendSingle{a});
+            if (nresolved) {
+#if SIGMA_CUDA
+                rt.launches++;
+                extend_single_k<<<1, 32, 0, rt.stream>>>(a);
+                ck(cudaGetLastError(), "launch");
+#else
+                rt.one(FExtendSingle{a});
+#endif
+            }
         } else if (nresolved) {
             if (nresolved >= 0xFFFFFFF0ull) throw std::runtime_error("witness stack too large for 32-bit positions");
             const u32 w = (u32)nresolved;
@@ -1804,9 +1814,7 @@ struct pf_sigma_ctx {
             key.reserve(rt, R + 1);
             ord.reserve(rt, R + 1);
             words.reserve(rt, R + 1);
-            fw.reserve(rt, nf);
-            rt.zero(fw.p, (size_t)nf * 8);
-            rt.each(FRecFid{c, rstart.p, R, w, key.p, ord.p, words.p, fw.p}, R);
+            rt.each(FRecFid{c, rstart.p, R, w, key.p, ord.p, words.p, nullptr}, R);
             k2.reserve(rt, R + 1);
             v2.reserve(rt, R + 1);
             radix_hist.reserve(rt, radix_hist_elems(R));
@@ -1815,16 +1823,19 @@ struct pf_sigma_ctx {
             const int bits = fid_bits();
             radix_sort_pairs(key.p, ord.p, k2.p, v2.p, R, bits, radix_hist.p, radix_hscan.p, scan_tmp32.p, rt.stream);
             rt.launches += 5 * (bits / 8);
-            frec.reserve(rt, nf + 1);
             ffirst.reserve(rt, nf + 1);
-            rt.zero(frec.p, (size_t)(nf + 1) * 4);
-            rt.each(FRecCount{c, rstart.p, frec.p}, R);
-            write_u32(ffirst.p + nf, scan32(frec.p, ffirst.p, nf));
+            rt.each(FExtendFirst{key.p, R, ffirst.p}, nf + 1);
             a.rec_start = rstart.p;
             a.rec_words = words.p;
             a.order = ord.p;
             a.f_first = ffirst.p;
+#if SIGMA_CUDA
+            rt.launches++;
+            extend_formula_k<<<(nf + EXT_WARPS - 1) / EXT_WARPS, EXT_WARPS * 32, 0, rt.stream>>>(a, nf);
+            ck(cudaGetLastError(), "launch");
+#else
             rt.each(FExtendFormula{a}, nf);
+#endif
         }
         check();
         if (!nf) {
