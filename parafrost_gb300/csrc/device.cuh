@@ -498,14 +498,17 @@ DEV bool grid_barrier(u32* bar, u32* err, const u32* snap_src = nullptr, u32* sn
             __threadfence();
             atomicAdd(&bar[1], 1u);
         } else {
-            const u64 t0 = global_ns();
-            while (vload(&bar[1]) == gen) {
-                if (global_ns() - t0 > kBarrierNs) {
+            // the clock is read every 64 looks only: a read takes longer than a look
+            u64 t0 = 0;
+            for (u32 k = 1; vload(&bar[1]) == gen; k++) {
+                if (k & 63u) continue;
+                const u64 t = global_ns();
+                if (!t0) t0 = t;
+                if (t - t0 > kBarrierNs) {
                     atomicOr(err, ERR_ITER);
                     ok = 0;
                     break;
                 }
-                __nanosleep(64);
             }
         }
         __threadfence();

@@ -49,7 +49,6 @@ struct LcveArgs {
     u64 pf = 0, pl = 0;   // L2 policies in the rounds kernel: streams go first, words last
     u32* cmin;            // per clause: the least rank of its graph vertices (MIS_NO_RANK when
                           // it has none or is deleted), built with the clause records
-    bool r0 = false;      // the first round's pull: walks test cmin instead of the neighbours
 };
 
 // write_scores (histogram.h:32-41): eligible[v-1] = v, scores[v] = ps*ns (32-bit wrap).
@@ -80,17 +79,16 @@ HD void k_rank(const LcveArgs& a, u32 p) {
     if (lcve_valid(a.c, v) && !lcve_freezable(a, v)) atom_min(&a.bound[2 * fid_of(a.c, v)], p);
 }
 
-// The independent set is decided in rounds of two phases:
-//   push: every vertex that went in during the last round marks its undecided
-//         higher-ranked neighbours out;
-//   pull: every undecided vertex walks its live clauses, from where its last walk
-//         stopped, looking at its lower-ranked graph neighbours; the first one
-//         that is not out stops the walk (the vertex stays undecided and resumes
-//         there), and a walk that reaches the end finds every lower neighbour out,
-//         so the vertex goes in.
+// The independent set is decided in rounds. In a round every undecided vertex walks its
+// live clauses, from where its last walk stopped, looking at its lower-ranked graph
+// neighbours; the first one that is not out stops the walk (the vertex stays undecided
+// and resumes there), and a walk that reaches the end finds every lower neighbour out,
+// so the vertex goes in and marks its undecided higher-ranked neighbours out.
 // A vertex goes in exactly when all its lower neighbours are out, and out when a
-// lower neighbour is in, as in the greedy walk in rank order. Out is final, so the
-// clauses a walk has passed never need another look. Vertices with more than
+// lower neighbour is in, as in the greedy walk in rank order. Both are final and true
+// whenever they are found, so the marks need no phase of their own and a walk may see
+// decisions of its own round: the set does not depend on the schedule. Out is final, so
+// the clauses a walk has passed never need another look. Vertices with more than
 // MIS_WARP_MIN_OCC clauses are walked by a whole warp; the others by one thread,
 // or by a group of lanes when few of them are left (mis_lanes).
 constexpr u32 MIS_WARP_MIN_OCC = 32;
@@ -192,11 +190,11 @@ struct MisCl {
     HD bool deleted() const { return !r0 && (q.w >> 31) != 0; }
     HD u32 size() const { return q.w & 0x7FFFFFFFu; }
 };
-HD MisCl mis_cl(const LcveArgs& a, u32 r) {
+HD MisCl mis_cl(const LcveArgs& a, u32 r, bool r0) {
     MisCl cl;
     cl.r = r;
-    cl.r0 = a.r0;
-    if (a.r0) {
+    cl.r0 = r0;
+    if (r0) {
         cl.q.x = ldro_hint(&a.cmin[r], a.pf);
         cl.q.y = cl.q.z = cl.q.w = 0;
     } else {
@@ -330,16 +328,16 @@ HD bool mis_blocked_in(const LcveArgs& a, u32 v, u32 rv, const MisCl& cl) {
 // Pull walk of undecided vertex v by one thread: true when v went in; otherwise the
 // resume point is stored (v stays undecided). The next clause's record is loaded
 // before the current one is examined.
-HD bool mis_pull_one(const LcveArgs& a, u32 v, u32 wv) {
+HD bool mis_pull_one(const LcveArgs& a, u32 v, u32 wv, bool r0) {
     const u32 rv = mis_rank(wv);
     const u32 p = V2L(v), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
     const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
     u32 t = vload(&a.resume[v]);
     if (t < n) {
-        MisCl cl = mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf));
+        MisCl cl = mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf), r0);
         for (; t < n; t++) {
             MisCl nx = cl;
-            if (t + 1 < n) nx = mis_cl(a, ldro_hint(&a.c.ot_refs[t + 1 < np ? op + t + 1 : on + t + 1], a.pf));
+            if (t + 1 < n) nx = mis_cl(a, ldro_hint(&a.c.ot_refs[t + 1 < np ? op + t + 1 : on + t + 1], a.pf), r0);
             if (mis_blocked_in(a, v, rv, cl)) {
                 a.resume[v] = t;
                 return false;
@@ -377,10 +375,10 @@ HD void mis_push_vertex(const LcveArgs& a, u32 u) {
     const u32 p = V2L(u), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
     const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
     if (!n) return;
-    MisCl cl = mis_cl(a, ldro_hint(&a.c.ot_refs[op], a.pf));
+    MisCl cl = mis_cl(a, ldro_hint(&a.c.ot_refs[op], a.pf), false);
     for (u32 t = 0; t < n; t++) {
         MisCl nx = cl;
-        if (t + 1 < n) nx = mis_cl(a, ldro_hint(&a.c.ot_refs[t + 1 < np ? op + t + 1 : on + t + 1], a.pf));
+        if (t + 1 < n) nx = mis_cl(a, ldro_hint(&a.c.ot_refs[t + 1 < np ? op + t + 1 : on + t + 1], a.pf), false);
         mis_push_clause(a, u, ru, cl);
         cl = nx;
     }
@@ -389,12 +387,12 @@ HD void mis_push_vertex(const LcveArgs& a, u32 u) {
 #if !SIGMA_CUDA
 // Serial rounds of the emulation build: the same phases over the same lists.
 HD void k_mis_push(const LcveArgs& a, const u32* in, u32 idx) { mis_push_vertex(a, in[idx]); }
-HD void k_mis_pull(const LcveArgs& a, const u32* in, const MisFront& und, const MisFront& ins, u32 idx) {
+HD void k_mis_pull(const LcveArgs& a, const u32* in, const MisFront& und, const MisFront& ins, bool r0, u32 idx) {
     const u32 v = in[idx];
     const u32 wv = a.word[v];
     if (mis_dec(wv) != MIS_UNDECIDED) return;
     const bool big = mis_is_big(a.c, v);
-    if (mis_pull_one(a, v, wv)) {
+    if (mis_pull_one(a, v, wv, r0)) {
         if (big) ins.big[atom_add(ins.nbig, 1u)] = v;
         else ins.small[atom_add(ins.nsmall, 1u)] = v;
     } else {
@@ -403,27 +401,34 @@ HD void k_mis_pull(const LcveArgs& a, const u32* in, const MisFront& und, const 
     }
 }
 #else
-// All rounds in one cooperative launch. Round r reads the undecided and new-in
-// lists u[r&1], in[r&1] (lengths in counter set r%3: undecided small, large, in
-// small, large) and writes u[(r+1)&1], in[(r+1)&1] through counter set (r+1)%3;
-// set (r+2)%3, last read in round r-1, is cleared for round r+1. Grid barriers
-// separate the push phase, the pull phase and the rounds.
+// All rounds in one cooperative launch. Round r reads the undecided lists u[r&1]
+// (lengths in counter set r%3: small, large) and writes u[(r+1)&1] through counter set
+// (r+1)%3; set (r+2)%3, last read in round r-1, is cleared for round r+1. One grid
+// barrier ends a round.
+//
+// What bounds a small election is the chain of dependent decisions: a round costs the
+// barrier and some five dependent loads whatever its size. So once every undecided
+// vertex has its own lanes (us * lanes <= threads), a group keeps its vertex and tries
+// again up to MIS_TRIES times before the round ends, and sees its neighbours' decisions
+// as they are made. Device time of a round's elections, before (a push phase and a pull
+// phase a round, two barriers) and now: 200 variables 507 and 88 us (18 and 8 rounds),
+// 10k-variable 3-SAT 739 and 141, 1M mixed clauses 1245 and 740, a 6.8M-clause AIG 3449
+// and 2830 (50 and 23 rounds), 80M community clauses 10.9 and 8.1 ms.
 struct MisRounds {
     u32* u_small[2];
     u32* u_big[2];
-    u32* in_small[2];
-    u32* in_big[2];
-    u32* ctr;        // three sets of four counters
+    u32* ctr;        // three sets of four counters (two used)
     u32* bar;        // grid barrier: [0] arrivals, [1] generation
     u32* rounds;     // out: rounds run
     u32 max_rounds;
-    u32* trace;      // optional: per round [undecided small, big, went-in small, big, start ns / 1024]
+    u32* trace;      // optional: per round [undecided small, big, start ns / 1024]
     u32 trace_cap;   // rounds the trace holds
 };
+constexpr u32 MIS_TRIES = 48;
 
-// Vertices leaving a pull phase are staged per block in shared memory and copied
-// to the next lists with one reservation per block (a vertex that finds its
-// block's queue full goes to the list directly).
+// Vertices that stay undecided are staged per block in shared memory and copied to the
+// next lists with one reservation per block (a vertex that finds its block's queue full
+// goes to the list directly).
 constexpr u32 MIS_QCAP = 1024;
 
 struct MisBlockQueue {
@@ -487,21 +492,62 @@ DEV void mis_queue_flush(MisBlockQueue& q, const MisFront& f) {
     if (threadIdx.x == 0) q.ns = q.nb = 0;
 }
 
+// One try at vertex v by the lanes of mask gm (sub: this lane's place among the L of
+// them): clauses from `at` on, L at a time in list order, the first blocking one of a
+// step (lowest lane) stops the walk. Returns true when v is decided; a walk that
+// reaches the end puts v in and marks its neighbours out, the lanes sharing the clauses.
+DEV bool mis_try(const LcveArgs& a, u32 v, u32 gm, u32 gbase, u32 sub, u32 L, u32& at, bool r0) {
+    const u32 wv = vload(&a.word[v]);  // the same word for the whole group
+    if (mis_dec(wv) != MIS_UNDECIDED) return true;
+    const u32 rv = mis_rank(wv);
+    const u32 p = V2L(v), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
+    const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
+    for (u32 b0 = at; b0 < n; b0 += L) {
+        const u32 t = b0 + sub;
+        const bool blk = t < n && mis_blocked_in(a, v, rv, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf), r0));
+        const u32 m = (__ballot_sync(gm, blk) & gm) >> gbase;
+        if (m) {
+            at = b0 + (u32)(__ffs(m) - 1);
+            return false;
+        }
+    }
+    if (sub == 0) atomicOr(&a.word[v], mis_dec_bits(MIS_IN));
+    for (u32 t = sub; t < n; t += L)
+        mis_push_clause(a, v, rv, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf), false));
+    return true;
+}
+
+// The block marks out the neighbours of the vertices it put in (queue q, n of them),
+// eight lanes a vertex.
+DEV void mis_push_queue(const LcveArgs& a, const u32* q, u32 n) {
+    const u32 sub = threadIdx.x & 7u;
+    for (u32 k = threadIdx.x >> 3; k < n; k += blockDim.x >> 3) {
+        const u32 u = q[k];
+        const u32 ru = mis_rank(vload(&a.word[u]));
+        const u32 p = V2L(u), np = a.c.ot_size[p], m = np + a.c.ot_size[p + 1];
+        const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
+        for (u32 t = sub; t < m; t += 8)
+            mis_push_clause(a, u, ru, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf), false));
+    }
+}
+
 __global__ void __launch_bounds__(256, 6) mis_rounds_k(LcveArgs a0, MisRounds w) {
     LcveArgs a = a0;
     a.pf = l2_policy_first();
     a.pl = l2_policy_last();
-    __shared__ MisBlockQueue qu, qi;
+    __shared__ MisBlockQueue qu;
+    __shared__ u32 qin[MIS_QCAP];
+    __shared__ u32 nin;
     const u32 tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const u32 lane = threadIdx.x & 31u, nwarps = nth >> 5;
-    if (threadIdx.x == 0) qu.ns = qu.nb = qi.ns = qi.nb = 0;
+    if (threadIdx.x == 0) qu.ns = qu.nb = nin = 0;
     __syncthreads();
     for (u32 r = 0;; r++) {
-        a.r0 = r == 0;
+        // In the first round no vertex is out yet, so the walks test one word per clause.
+        const bool r0 = r == 0;
         const u32 cur = r % 3, nxt = (r + 1) % 3, old = (r + 2) % 3;
         const u32 us = vload(&w.ctr[4 * cur]), ub = vload(&w.ctr[4 * cur + 1]);
-        const u32 is = vload(&w.ctr[4 * cur + 2]), ib = vload(&w.ctr[4 * cur + 3]);
-        if (!us && !ub && !is && !ib) {
+        if (!us && !ub) {
             if (tid == 0) *w.rounds = r;
             return;
         }
@@ -510,143 +556,100 @@ __global__ void __launch_bounds__(256, 6) mis_rounds_k(LcveArgs a0, MisRounds w)
             return;
         }
         if (tid == 0)
-            for (u32 k = 0; k < 4; k++) w.ctr[4 * old + k] = 0;
+            for (u32 k = 0; k < 2; k++) w.ctr[4 * old + k] = 0;
         if (tid == 0 && w.trace && r < w.trace_cap) {
-            u32* t = w.trace + 5 * r;
+            u32* t = w.trace + 3 * r;
             t[0] = us;
             t[1] = ub;
-            t[2] = is;
-            t[3] = ib;
-            t[4] = (u32)(global_ns() >> 10);
+            t[2] = (u32)(global_ns() >> 10);
         }
-        // push: the vertices that went in last round (lists written by other blocks: uncached reads)
-        const u32* pin_b = w.in_big[r & 1];
-        for (u32 idx = tid >> 5; idx < ib; idx += nwarps) {
-            const u32 u = vload(&pin_b[idx]);
-            const u32 ru = mis_rank(a.word[u]);
-            const u32 p = V2L(u), np = a.c.ot_size[p], nn = a.c.ot_size[p + 1];
-            const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1];
-            for (u32 t = lane; t < np + nn; t += 32)
-                mis_push_clause(a, u, ru, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + (t - np)], a.pf)));
-            __syncwarp();
-        }
-        const u32* pin_s = w.in_small[r & 1];
-        const u32 li = mis_lanes(is, nth);
-        if (li == 1) {
-            for (u32 idx = tid; idx < is; idx += nth) mis_push_vertex(a, vload(&pin_s[idx]));
-        } else {
-            // a group of li lanes per vertex, clauses strided over the group
-            const u32 sub = lane & (li - 1u);
-            for (u32 idx = tid / li; idx < is; idx += nth / li) {
-                const u32 u = vload(&pin_s[idx]);
-                const u32 ru = mis_rank(a.word[u]);
-                const u32 p = V2L(u), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
-                const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
-                for (u32 t = sub; t < n; t += li)
-                    mis_push_clause(a, u, ru, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf)));
-            }
-        }
-        if (!grid_barrier(w.bar, a.c.err)) return;
-        // pull: the undecided vertices
-        MisFront fu, fi;
-        fu.small = w.u_small[(r + 1) & 1];
+        MisFront fu;
+        const bool odd = r & 1;
+        fu.small = odd ? w.u_small[0] : w.u_small[1];
         fu.nsmall = &w.ctr[4 * nxt];
-        fu.big = w.u_big[(r + 1) & 1];
+        fu.big = odd ? w.u_big[0] : w.u_big[1];
         fu.nbig = &w.ctr[4 * nxt + 1];
-        fi.small = w.in_small[(r + 1) & 1];
-        fi.nsmall = &w.ctr[4 * nxt + 2];
-        fi.big = w.in_big[(r + 1) & 1];
-        fi.nbig = &w.ctr[4 * nxt + 3];
-        const u32* pu_b = w.u_big[r & 1];
-        for (u32 idx = tid >> 5; idx < ub; idx += nwarps) {
-            const u32 v = vload(&pu_b[idx]);
-            const u32 wv = vload(&a.word[v]);
-            if (mis_dec(wv) != MIS_UNDECIDED) continue;  // warp-uniform
-            const u32 rv = mis_rank(wv);
-            const u32 p = V2L(v), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
-            const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1];
-            u32 stop = NONE;
-            for (u32 b0 = vload(&a.resume[v]); b0 < n && stop == NONE; b0 += 32) {
-                const u32 t = b0 + lane;
-                const bool blk = t < n && mis_blocked_in(a, v, rv, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + (t - np)], a.pf)));
-                const u32 m = __ballot_sync(0xffffffffu, blk);
-                if (m) stop = b0 + (u32)(__ffs(m) - 1);
-            }
-            if (lane == 0) {
-                if (stop != NONE) {
-                    a.resume[v] = stop;
-                    mis_queue_push(qu, fu, true, v);
-                } else {
-                    atomicOr(&a.word[v], mis_dec_bits(MIS_IN));
-                    mis_queue_push(qi, fi, true, v);
-                }
-            }
-            __syncwarp();
-        }
-        const u32* pu_s = w.u_small[r & 1];
+        // (lists written by other blocks: uncached reads)
+        const u32* pu_b = odd ? w.u_big[1] : w.u_big[0];
+        const u32* pu_s = odd ? w.u_small[1] : w.u_small[0];
         const u32 lu = mis_lanes(us, nth);
-        if (lu == 1) {
-            // warp-uniform trip count: the appends below take every lane
-            for (u32 base = tid - lane; base < us; base += nth) {
-                const u32 idx = base + lane;
-                u32 v = 0;
-                bool in = false, und = false;
-                if (idx < us) {
-                    v = vload(&pu_s[idx]);
-                    const u32 wv = vload(&a.word[v]);
-                    if (mis_dec(wv) == MIS_UNDECIDED) {
-                        in = mis_pull_one(a, v, wv);
-                        und = !in;
-                    }
-                }
-                mis_queue_warp(qi.small, qi.ns, fi.small, fi.nsmall, in, v);
-                mis_queue_warp(qu.small, qu.ns, fu.small, fu.nsmall, und, v);
+        const u32 sub = lane & (lu - 1u), gbase = lane - sub;
+        const u32 gm = lu == 32u ? kFull : ((1u << lu) - 1u) << gbase;
+        const u32 warp = tid >> 5;
+        if (!r0 && (u64)us * lu <= nth && ub <= nwarps) {
+            // every undecided vertex has its own lanes: try until it is decided
+            const bool hb = warp < ub, hs = tid / lu < us;
+            const u32 vb = hb ? vload(&pu_b[warp]) : 0u, vs = hs ? vload(&pu_s[tid / lu]) : 0u;
+            u32 ab = hb ? vload(&a.resume[vb]) : 0u, as = hs ? vload(&a.resume[vs]) : 0u;
+            bool wb = hb, ws = hs;
+            for (u32 k = 0; k < MIS_TRIES && __any_sync(kFull, wb || ws); k++) {
+                if (wb) wb = !mis_try(a, vb, kFull, 0, lane, 32, ab, false);  // warp-uniform
+                if (ws) ws = !mis_try(a, vs, gm, gbase, sub, lu, as, false);  // group-uniform
+                __syncwarp();
             }
+            if (wb && lane == 0) {
+                a.resume[vb] = ab;
+                mis_queue_push(qu, fu, true, vb);
+            }
+            if (ws && sub == 0) a.resume[vs] = as;
+            mis_queue_warp(qu.small, qu.ns, fu.small, fu.nsmall, ws && sub == 0, vs);
         } else {
-            // a group of lu lanes per vertex: batches of lu clauses in list order,
-            // the first blocking clause of a batch (lowest lane) stops the walk
-            const u32 sub = lane & (lu - 1u), gbase = lane - sub;
-            const u32 gmask = lu == 32u ? kFull : ((1u << lu) - 1u) << gbase;
-            const u32 gpw = 32u / lu;
-            for (u32 base = (tid >> 5) * gpw; base < us; base += nwarps * gpw) {
-                const u32 idx = base + lane / lu;
-                u32 v = 0;
-                bool in = false, und = false;
-                if (idx < us) {
-                    v = vload(&pu_s[idx]);
-                    const u32 wv = vload(&a.word[v]);
-                    if (mis_dec(wv) == MIS_UNDECIDED) {  // the same word for the whole group
-                        const u32 rv = mis_rank(wv);
-                        const u32 p = V2L(v), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
-                        const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
-                        u32 stop = NONE;
-                        for (u32 b0 = vload(&a.resume[v]); b0 < n; b0 += lu) {
-                            const u32 t = b0 + sub;
-                            const bool blk =
-                                t < n && mis_blocked_in(a, v, rv, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf)));
-                            const u32 m = (__ballot_sync(gmask, blk) & gmask) >> gbase;
-                            if (m) {
-                                stop = b0 + (u32)(__ffs(m) - 1);
-                                break;
-                            }
-                        }
-                        if (sub == 0) {
-                            if (stop != NONE) {
-                                a.resume[v] = stop;
-                                und = true;
-                            } else {
-                                atom_or(&a.word[v], mis_dec_bits(MIS_IN));
-                                in = true;
-                            }
+            for (u32 idx = warp; idx < ub; idx += nwarps) {
+                const u32 v = vload(&pu_b[idx]);
+                u32 at = vload(&a.resume[v]);
+                const bool und = !mis_try(a, v, kFull, 0, lane, 32, at, r0);
+                if (und && lane == 0) {
+                    a.resume[v] = at;
+                    mis_queue_push(qu, fu, true, v);
+                }
+                __syncwarp();
+            }
+            if (lu == 1) {
+                // one thread a vertex; the block's own new in vertices are staged and their
+                // neighbours marked by all its threads (block-uniform trip count)
+                for (u32 base = blockIdx.x * blockDim.x; base < us; base += nth) {
+                    const u32 idx = base + threadIdx.x;
+                    u32 v = 0;
+                    bool in = false, und = false;
+                    if (idx < us) {
+                        v = vload(&pu_s[idx]);
+                        const u32 wv = vload(&a.word[v]);
+                        if (mis_dec(wv) == MIS_UNDECIDED) {
+                            in = mis_pull_one(a, v, wv, r0);
+                            und = !in;
                         }
                     }
+                    mis_queue_warp(qu.small, qu.ns, fu.small, fu.nsmall, und, v);
+                    const u32 k = warp_append(&nin, in);
+                    if (in) qin[k] = v;
+                    __syncthreads();
+                    const u32 n = nin;
+                    __syncthreads();
+                    if (n > MIS_QCAP - 256u || base + nth >= us) {
+                        mis_push_queue(a, qin, n);
+                        if (threadIdx.x == 0) nin = 0;
+                        __syncthreads();
+                    }
                 }
-                mis_queue_warp(qi.small, qi.ns, fi.small, fi.nsmall, in, v);
-                mis_queue_warp(qu.small, qu.ns, fu.small, fu.nsmall, und, v);
+            } else {
+                // a group of lu lanes a vertex
+                const u32 gpw = 32u / lu;
+                for (u32 base = warp * gpw; base < us; base += nwarps * gpw) {
+                    const u32 idx = base + lane / lu;
+                    u32 v = 0;
+                    bool und = false;
+                    if (idx < us) {
+                        v = vload(&pu_s[idx]);
+                        u32 at = vload(&a.resume[v]);
+                        und = !mis_try(a, v, gm, gbase, sub, lu, at, r0);
+                        if (und && sub == 0) a.resume[v] = at;
+                        und = und && sub == 0;
+                    }
+                    mis_queue_warp(qu.small, qu.ns, fu.small, fu.nsmall, und, v);
+                }
             }
         }
         mis_queue_flush(qu, fu);
-        mis_queue_flush(qi, fi);
         if (!grid_barrier(w.bar, a.c.err)) return;
     }
 }

@@ -54,8 +54,8 @@ struct FMisRec { LcveArgs a; Q4* rec; HD void operator()(u32 i) const { k_mis_re
 #if !SIGMA_CUDA
 struct FMisPush { LcveArgs a; const u32* in; HD void operator()(u32 i) const { k_mis_push(a, in, i); } };
 struct FMisPull {
-    LcveArgs a; const u32* in; MisFront und, ins;
-    HD void operator()(u32 i) const { k_mis_pull(a, in, und, ins, i); }
+    LcveArgs a; const u32* in; MisFront und, ins; bool r0;
+    HD void operator()(u32 i) const { k_mis_pull(a, in, und, ins, r0, i); }
 };
 #endif
 struct FMisInit { LcveArgs a; MisFront b; HD void operator()(u32 i) const { k_mis_init(a, b, i); } };
@@ -341,7 +341,9 @@ struct pf_sigma_ctx {
     DBuf<u32> score, order, order_k2, order_v2, rank, bound, pvs, flags, flags_scan;
     DBuf<u32> mis_big_a, mis_big_b;
     DBuf<u32> mis_word, mis_resume, mis_cmin;
-    DBuf<u32> mis_in[4];  // new-in lists of the election rounds (small x2, large x2)
+#if !SIGMA_CUDA
+    DBuf<u32> mis_in[4];  // new-in lists of the serial election rounds (small x2, large x2)
+#endif
     DBuf<Q4> mis_rec;  // the election's 16-byte clause records
     DBuf<u32> mis_gbits;  // the election's graph membership bitmap
     DBuf<u32> pv_perm, pv_key;
@@ -506,7 +508,14 @@ struct pf_sigma_ctx {
         }
         return cache;
     }
-    int mis_rounds_grid() { return coop_grid(mis_rounds_k, mis_grid); }
+    // Sixteen threads a variable at most: a grid barrier costs an arrival per block, and
+    // a small election is a chain of barriers. Measured over an election's share of a
+    // round: 200 variables 139 us at the full grid, 88 at 16 a variable, 121 at 4; 10k
+    // variables 180, 141 and 195; from 100k variables on the grid is full at 4 or more
+    // (100k: 469, 471, 469).
+    int mis_rounds_grid() {
+        return (int)std::min<u64>((u64)coop_grid(mis_rounds_k, mis_grid), ((u64)nvars * 16 + 255) / 256);
+    }
 #endif
     void write_u64(u64* d, u64 v) { rt.h2d(d, &v, 8); }
 
@@ -786,21 +795,20 @@ struct pf_sigma_ctx {
 #if SIGMA_CUDA
     // Traces of the persistent launches, printed to stderr when the environment sets
     // PF_TRACE: per propagation wave the pending literals, the clauses collected (or
-    // "sweep") and the wave's device time; per election round the undecided and
-    // went-in vertex lists (small and big adjacency) and the round's device time.
+    // "sweep") and the wave's device time; per election round the undecided vertex
+    // lists (small and big adjacency) and the round's device time.
     static constexpr u32 kPropTraceWaves = 4096;
     const bool trace_on = std::getenv("PF_TRACE") != nullptr;
     DBuf<u32> prop_trace;
     DBuf<u64> prop_parts;
     void print_mis_trace(u32 rounds) {
         const u32 n = std::min(rounds, kPropTraceWaves);
-        std::vector<u32> t(5 * (size_t)n + 5);
-        if (n) rt.d2h(t.data(), prop_trace.p, 5 * (size_t)n * 4);
+        std::vector<u32> t(3 * (size_t)n + 3);
+        if (n) rt.d2h(t.data(), prop_trace.p, 3 * (size_t)n * 4);
         std::fprintf(stderr, "election phase %u: %u rounds\n", phase, rounds);
         for (u32 i = 0; i < n; i++) {
-            const double us = i + 1 < n ? (double)(u32)(t[5 * i + 9] - t[5 * i + 4]) * 1.024 : 0.0;
-            std::fprintf(stderr, "  round %u undecided %u+%u in %u+%u %.1f us\n", i, t[5 * i], t[5 * i + 1],
-                         t[5 * i + 2], t[5 * i + 3], us);
+            const double us = i + 1 < n ? (double)(u32)(t[3 * i + 5] - t[3 * i + 2]) * 1.024 : 0.0;
+            std::fprintf(stderr, "  round %u undecided %u+%u %.1f us\n", i, t[3 * i], t[3 * i + 1], us);
         }
     }
     void print_prop_trace(u32 waves) {
@@ -953,11 +961,13 @@ struct pf_sigma_ctx {
         rt.launches += 5 * (bits / 8);
         rt.zero(bound.p, (size_t)nform * 8, 0xFF);
         rt.each(FRank{a}, nvars);
-        // Independent set by push/pull rounds. Undecided lists: flags|mis_big_a and
-        // flags_scan|mis_big_b; new-in lists: mis_in[0..3].
+        // Independent set by rounds. Undecided lists: flags|mis_big_a and
+        // flags_scan|mis_big_b.
         mis_big_a.reserve(rt, nvars + 1);
         mis_big_b.reserve(rt, nvars + 1);
+#if !SIGMA_CUDA
         for (auto& b : mis_in) b.reserve(rt, nvars + 1);
+#endif
         u32* ctr = counters.p + 12;  // [12..23] three sets of list lengths, [24..25] barrier, [26] rounds
         rt.zero(ctr, 15 * 4);
 #if SIGMA_CUDA
@@ -984,10 +994,6 @@ struct pf_sigma_ctx {
         w.u_small[1] = flags_scan.p;
         w.u_big[0] = mis_big_a.p;
         w.u_big[1] = mis_big_b.p;
-        w.in_small[0] = mis_in[0].p;
-        w.in_small[1] = mis_in[1].p;
-        w.in_big[0] = mis_in[2].p;
-        w.in_big[1] = mis_in[3].p;
         w.ctr = ctr;
         w.bar = ctr + 12;
         w.rounds = ctr + 14;
@@ -1018,10 +1024,9 @@ struct pf_sigma_ctx {
             if (n[2]) rt.each(FMisPush{a, ins[cur].small}, n[2]);
             if (n[3]) rt.each(FMisPush{a, ins[cur].big}, n[3]);
             rt.zero(ctr + 4 * (cur ^ 1u), 16);
-            LcveArgs ar = a;
-            ar.r0 = rounds == 1;  // the first round's walks test the clauses' least ranks
-            if (n[0]) rt.each(FMisPull{ar, und[cur].small, und[cur ^ 1u], ins[cur ^ 1u]}, n[0]);
-            if (n[1]) rt.each(FMisPull{ar, und[cur].big, und[cur ^ 1u], ins[cur ^ 1u]}, n[1]);
+            const bool r0 = rounds == 1;  // the first round's walks test the clauses' least ranks
+            if (n[0]) rt.each(FMisPull{a, und[cur].small, und[cur ^ 1u], ins[cur ^ 1u], r0}, n[0]);
+            if (n[1]) rt.each(FMisPull{a, und[cur].big, und[cur ^ 1u], ins[cur ^ 1u], r0}, n[1]);
         }
         kclock[K_MIS].stop(rt);
 #endif
@@ -2795,7 +2800,9 @@ void pf_sigma_destroy(pf_sigma_ctx* ctx) {
     c.mis_word.free();
     c.mis_resume.free();
     c.mis_cmin.free();
+#if !SIGMA_CUDA
     for (auto& b : c.mis_in) b.free();
+#endif
     c.mis_rec.free();
     c.mis_gbits.free();
     c.down_learnt.free();
