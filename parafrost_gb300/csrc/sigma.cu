@@ -784,17 +784,21 @@ struct pf_sigma_ctx {
 
     // The mean occurrence-list length (literals in use per literal slot) times the
     // sweep divisor, 0 when sweeps are off (prop_use_sweep).
+    // (The divisor: a sweep reads the whole store, a walk a few random sectors an entry.
+    // Propagation of the 80M-clause community formula at 1/2, 1/4, 1/8, 1/16 and 1/64 of
+    // the store: 13.5, 9.6, 8.7, 8.5 and 9.0 ms.)
+    u32 sweep_div() const { return opt.sweep_div > 0 ? (u32)opt.sweep_div : 16u; }
     u32 sweep_scale() const {
         if (opt.sweep_div < 0) return 0;
-        const u64 div = opt.sweep_div ? (u64)opt.sweep_div : 64ull;
-        return (u32)std::min<u64>(std::max<u64>(div * nlits_used / std::max<u32>(D, 1), 1), 0xFFFFFFFFull);
+        const u64 mean = (u64)sweep_div() * nlits_used / std::max<u32>(D, 1);
+        return (u32)std::min<u64>(std::max<u64>(mean, 1), 0xFFFFFFFFull);
     }
     // Blocks of the per-variable warp kernels.
     u32 pv_grid() const { return (u32)rt.sms * (opt.pv_blocks > 0 ? (u32)opt.pv_blocks : 8u); }
 
 #if SIGMA_CUDA
     // Traces of the persistent launches, printed to stderr when the environment sets
-    // PF_TRACE: per propagation wave the pending literals, the clauses collected (or
+    // PF_TRACE: per propagation wave the pending literals, the list parts (and
     // "sweep") and the wave's device time; per election round the undecided vertex
     // lists (small and big adjacency) and the round's device time.
     static constexpr u32 kPropTraceWaves = 4096;
@@ -813,19 +817,14 @@ struct pf_sigma_ctx {
     }
     void print_prop_trace(u32 waves) {
         const u32 n = std::min(waves, kPropTraceWaves);
-        std::vector<u32> t(4 * (size_t)n + 4);
-        if (n) rt.d2h(t.data(), prop_trace.p, 4 * (size_t)n * 4);
+        std::vector<u32> t(3 * (size_t)n + 3);
+        if (n) rt.d2h(t.data(), prop_trace.p, 3 * (size_t)n * 4);
         std::fprintf(stderr, "prop phase %u: %u waves, ncls %u\n", phase, waves, ncls);
         for (u32 i = 0; i < n; i++) {
-            const u32* w = &t[4 * i];
-            const double us = i + 1 < n ? (double)(u32)(w[6] - w[2]) * 1.024 : 0.0;
-            if (w[1] >> 31) {
-                std::fprintf(stderr, "  wave %u pending %u sweep %.1f us\n", i, w[0], us);
-            } else {
-                const double la = w[3] ? (double)(u32)(w[3] - w[2]) * 1.024 : 0.0;
-                std::fprintf(stderr, "  wave %u pending %u collected %u %.1f us (lists %.1f us)\n", i, w[0], w[1], us,
-                             la);
-            }
+            const u32* w = &t[3 * i];
+            const double us = i + 1 < n ? (double)(u32)(w[5] - w[2]) * 1.024 : 0.0;
+            std::fprintf(stderr, "  wave %u pending %u parts %u%s %.1f us\n", i, w[0], w[1] & 0x7FFFFFFFu,
+                         w[1] >> 31 ? " sweep" : "", us);
         }
     }
 #endif
@@ -833,12 +832,7 @@ struct pf_sigma_ctx {
     // prop (elimination.cpp:64-99).
     void prop() {
         if (prop_head >= ntrail) return;
-#if SIGMA_CUDA
-        // collected clauses plus the free slots of the warps' closed runs (at most 31
-        // per run of PROP_SLOTS, and two partly used runs per warp and wave)
-        const size_t nwarps = (size_t)rt.sms * 4 * 256 / 32;
-        work.reserve(rt, (size_t)ot_refs.n + ot_refs.n / 8 + 2 * nwarps * PROP_SLOTS + 1024);
-#else
+#if !SIGMA_CUDA
         work.reserve(rt, (size_t)std::max<u64>(ot_refs.n, 1024));
 #endif
         if (cl_stamp.n < hdr.n) {
@@ -853,21 +847,32 @@ struct pf_sigma_ctx {
             a.head = prop_head;
             a.stamp = wave_stamp + 1;
             a.cl_stamp = cl_stamp.p;
-            a.work = work.p;
-            a.nwork = nullptr;
-            a.cap_work = (u32)work.n;
-            // parts of long lists: at most one per PROP_PART occurrences of the table
-            prop_parts.reserve(rt, (size_t)(nlits_used / PROP_PART) + 1024);
-            PropWaves w{counters.p + 22, counters.p + 24, counters.p + 26, loop_bound(), sweep_scale(),
-                        nullptr, 0, counters.p + 28, prop_parts.p, counters.p + 29, (u32)prop_parts.n};
+            a.work = a.nwork = nullptr;  // (the serial waves' collected clauses)
+            a.cap_work = 0;
+            // parts of long lists: a literal's lists are cut once, so all waves together
+            // make at most one part per PROP_PART occurrences of the table
+            const size_t nparts = (size_t)(nlits_used / PROP_PART) + 1024;
+            prop_parts.reserve(rt, 2 * nparts);
+            PropWaves w{};
+            w.tail = counters.p + 18;
+            w.pend[0] = flags.p;  // nvars + 1 words each: a literal is pending once
+            w.pend[1] = flags_scan.p;
+            w.parts[0] = prop_parts.p;
+            w.parts[1] = prop_parts.p + nparts;
+            w.cap_parts = (u32)nparts;
+            w.ctr = counters.p + 12;
+            w.bar = counters.p + 24;
+            w.waves = counters.p + 26;
+            w.max_waves = loop_bound();
+            w.sweep_scale = sweep_scale();
+            w.sweep_div = sweep_div();
             if (trace_on) {
                 prop_trace.reserve(rt, 5 * kPropTraceWaves);
                 w.trace = prop_trace.p;
                 w.trace_cap = kPropTraceWaves - 1;
             }
-            rt.zero(counters.p + 22, 5 * 4);  // [22..23] work counters, [24..25] barrier, [26] waves
-            rt.d2d(counters.p + 28, counters.p + 0, 4);  // [28] the trail's end for the first wave
-            rt.zero(counters.p + 29, 2 * 4);             // [29..30] list-part counters
+            rt.zero(counters.p + 12, 15 * 4);  // [12..17] wave counters, [24..25] barrier, [26] waves
+            rt.d2d(counters.p + 18, counters.p + 0, 4);  // [18] the trail's end for the first wave
             void* args[] = {&a, &w};
             rt.launches++;
             // four blocks per SM: most waves of a propagation are small, and the grid
@@ -875,12 +880,14 @@ struct pf_sigma_ctx {
             ck(cudaLaunchCooperativeKernel((const void*)prop_waves_k, dim3(rt.sms * 4), dim3(256), args, 0,
                                            rt.stream),
                "cooperative launch");
-            check();
-            const u32 waves = read_u32(counters.p + 26);
+            word_to(counters.p + 26, 0);
+            word_to(counters.p + 0, 1);
+            read_slots_checked();
+            const u32 waves = (u32)hr[0];
             if (trace_on) print_prop_trace(waves);
-            wave_stamp += waves;
+            wave_stamp += waves + 1;
             prop_waves += waves;
-            ntrail = read_u32(counters.p + 0);
+            ntrail = (u32)hr[1];
             prop_head = ntrail;
         }
 #else
