@@ -66,6 +66,25 @@ __global__ void single_k(F f) {
 }
 #endif
 
+// Up to eight device values (slot k: `words` 32-bit words at src, at most two, or a sum
+// of 64-bit pairs; no source: 0) that the host reads together.
+struct ReadSlots {
+    const void* src[8] = {};
+    u32 words[8] = {};
+};
+HD u64 read_slot(const ReadSlots& s, u32 k) {
+    if (!s.src[k]) return 0;
+    if (s.words[k] == 1) return *(const u32*)s.src[k];
+    u64 t = 0;
+    for (u32 i = 0; i < s.words[k] / 2; i++) t += ((const u64*)s.src[k])[i];
+    return t;
+}
+#if SIGMA_CUDA
+__global__ void read_slots_k(ReadSlots s, u64* out) {
+    if (threadIdx.x < 8) out[threadIdx.x] = read_slot(s, threadIdx.x);
+}
+#endif
+
 struct Runtime {
     Stream stream = nullptr;
     int sms = 152;
@@ -73,7 +92,16 @@ struct Runtime {
     size_t budget = 0;  // 0 = no limit
     unsigned launches = 0;
     unsigned syncs = 0;  // host waits for the device (synchronous reads, stream and event syncs)
+    // page-locked host memory that short reads go through: a copy to pageable memory is
+    // staged by the driver
+    static constexpr size_t kPinBytes = 4096;
+    void* pin = nullptr;
 
+    void init_pin() {
+#if SIGMA_CUDA
+        ck(cudaMallocHost(&pin, kPinBytes), "host alloc");
+#endif
+    }
     void init() {
 #if SIGMA_CUDA
         int dev = 0;
@@ -85,6 +113,8 @@ struct Runtime {
     void destroy() {
 #if SIGMA_CUDA
         if (stream) cudaStreamDestroy(stream);
+        if (pin) cudaFreeHost(pin);
+        pin = nullptr;
         stream = nullptr;
 #endif
     }
@@ -135,8 +165,10 @@ struct Runtime {
         if (!b) return;
         syncs++;
 #if SIGMA_CUDA
-        ck(cudaMemcpyAsync(h, d, b, cudaMemcpyDeviceToHost, stream), "d2h");
+        void* to = pin && b <= kPinBytes ? pin : h;
+        ck(cudaMemcpyAsync(to, d, b, cudaMemcpyDeviceToHost, stream), "d2h");
         ck(cudaStreamSynchronize(stream), "sync");
+        if (to != h) std::memcpy(h, to, b);
 #else
         std::memcpy(h, d, b);
 #endif
@@ -210,11 +242,31 @@ struct Runtime {
     }
 };
 
+// Device array, released with its owner (or by free()).
 template <class T>
 struct DBuf {
     T* p = nullptr;
     size_t n = 0;
     Runtime* rt = nullptr;
+    DBuf() = default;
+    DBuf(const DBuf&) = delete;
+    DBuf& operator=(const DBuf&) = delete;
+    DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), rt(o.rt) {
+        o.p = nullptr;
+        o.n = 0;
+    }
+    DBuf& operator=(DBuf&& o) noexcept {
+        if (this != &o) {
+            free();
+            p = o.p;
+            n = o.n;
+            rt = o.rt;
+            o.p = nullptr;
+            o.n = 0;
+        }
+        return *this;
+    }
+    ~DBuf() { free(); }
     void reserve(Runtime& r, size_t count) {
         rt = &r;
         if (count <= n && p) return;
@@ -241,7 +293,6 @@ struct DBuf {
     size_t bytes() const { return n * sizeof(T); }
 };
 
-// Device-time stage timer (CUDA events on the context stream; wall clock in emulation).
 // Device time of one kernel over a round: an event pair around each launch, read
 // once after the round has finished (no synchronisation per launch).
 struct KernelClock {
@@ -304,45 +355,64 @@ struct KernelClock {
     }
 };
 
-struct StageTimer {
+// Device times of the stages of a round: event pairs with a stage and a phase each,
+// read once after the round has finished (wall clock in emulation).
+struct StageClock {
+    struct Span { int stage, phase; };
+    std::vector<Span> spans;
 #if SIGMA_CUDA
-    cudaEvent_t a = nullptr, b = nullptr;
+    std::vector<cudaEvent_t> ev;
 #else
+    std::vector<double> ms;
     std::chrono::steady_clock::time_point t0;
 #endif
-    void init() {
-#if SIGMA_CUDA
-        cudaEventCreate(&a);
-        cudaEventCreate(&b);
-#endif
-    }
-    void destroy() {
-#if SIGMA_CUDA
-        if (a) cudaEventDestroy(a);
-        if (b) cudaEventDestroy(b);
-        a = b = nullptr;
-#endif
-    }
     void start(Runtime& rt) {
 #if SIGMA_CUDA
-        cudaEventRecord(a, rt.stream);
+        while (2 * spans.size() + 2 > ev.size()) {
+            cudaEvent_t e;
+            ck(cudaEventCreate(&e), "event");
+            ev.push_back(e);
+        }
+        ck(cudaEventRecord(ev[2 * spans.size()], rt.stream), "event");
 #else
         (void)rt;
         t0 = std::chrono::steady_clock::now();
 #endif
     }
-    double stop(Runtime& rt) {
-        rt.syncs++;
+    void stop(Runtime& rt, int stage, int phase) {
 #if SIGMA_CUDA
-        cudaEventRecord(b, rt.stream);
-        cudaEventSynchronize(b);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, a, b);
-        return ms;
+        ck(cudaEventRecord(ev[2 * spans.size() + 1], rt.stream), "event");
 #else
         (void)rt;
-        return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+        ms.push_back(std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
 #endif
+        spans.push_back(Span{stage, phase});
+    }
+    // f(span, ms) for every finished span; the stream must have finished them.
+    template <class F>
+    void each(F f) const {
+        for (size_t i = 0; i < spans.size(); i++) {
+#if SIGMA_CUDA
+            float t = 0;
+            ck(cudaEventElapsedTime(&t, ev[2 * i], ev[2 * i + 1]), "event time");
+            f(spans[i], (double)t);
+#else
+            f(spans[i], ms[i]);
+#endif
+        }
+    }
+    void reset() {
+        spans.clear();
+#if !SIGMA_CUDA
+        ms.clear();
+#endif
+    }
+    void destroy() {
+#if SIGMA_CUDA
+        for (cudaEvent_t e : ev) cudaEventDestroy(e);
+        ev.clear();
+#endif
+        spans.clear();
     }
 };
 

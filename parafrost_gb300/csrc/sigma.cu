@@ -309,7 +309,8 @@ enum Stage { ST_OT = 0, ST_PROP, ST_LCVE, ST_SORT, ST_SUB, ST_VE, ST_BCE, ST_ERE
 struct pf_sigma_ctx {
     pf_options opt;
     Runtime rt;
-    StageTimer tm;
+    StageClock tm;      // stage spans of the round
+    StageClock whole;   // the whole round
     // DRAT proof of the round (opt.proof): lines [n, lits...] written by the kernels
     // into `proof` at the device counter counters64[4] (units as they are assigned);
     // proof_bound bounds the words reserved so far
@@ -353,6 +354,12 @@ struct pf_sigma_ctx {
     DBuf<u64> big64a, big64b;
     DBuf<uint8_t> down_learnt;  // learnt flags of the downloaded clauses
     DBuf<u64> up_off;           // offsets of an upload from host buffers
+    DBuf<u64> up_first, up_base, up_cls;  // per formula of a batch upload
+    DBuf<u32> up_nv;
+    // batch results and model extension: records, units and values in formula order
+    DBuf<u32> rs_flag, rs_scan, rs_start, rs_key, rs_val, rs_k2, rs_v2, rs_out, rs_first;
+    DBuf<u64> rs_words, rs_size, rs_off, rs_fsum, rs_pfirst;
+    DBuf<uint8_t> rs_value, rs_packed;
     DBuf<uint8_t> up_learnt;    // learnt flags of an upload from host buffers
     DBuf<u32> big32a, big32b;
     // BVE
@@ -439,11 +446,12 @@ struct pf_sigma_ctx {
         return c;
     }
 
-    // Values the host needs together (scan totals, counters, the error word) are
-    // gathered into device slots on the stream and read back with one copy, so a
-    // stage waits for the device once instead of once per value.
-    DBuf<u64> hread;
+    // Values the host needs together (scan totals, counters, the error word) are named
+    // as slots and read at once: one kernel writes them to page-locked memory and the
+    // host waits once, instead of once (and once per copy) for every value.
+    DBuf<u64> hread;  // scan totals
     u64 hr[8] = {};
+    ReadSlots slots;
     u64* hslot(int k) {
         hread.reserve(rt, 8);
         return hread.p + k;
@@ -452,24 +460,47 @@ struct pf_sigma_ctx {
     template <class Tin, class T>
     void scan_to(const Tin* in, T* out, size_t n, int k) {
 #if SIGMA_CUDA
-        rt.zero(hslot(k), 8);
         scan1_launch(in, out, n, (T*)hslot(k));
 #else
-        u64 t;
+        T t;
         if constexpr (sizeof(T) == 4) t = scan32(in, out, n);
         else t = scan64(in, out, n);
-        rt.h2d(hslot(k), &t, 8);
+        rt.h2d(hslot(k), &t, sizeof t);
 #endif
+        slots.src[k] = hslot(k);
+        slots.words[k] = sizeof(T) / 4;
     }
-    // a device word into slot k (zero-extended)
+    // a device word, double word, or the sum of kSpreadSlots double words into slot k;
+    // the source keeps its value until the slots are read
     void word_to(const u32* d, int k) {
-        rt.zero(hslot(k), 8);
-        rt.d2d(hslot(k), d, 4);
+        slots.src[k] = d;
+        slots.words[k] = 1;
     }
-    // all slots into hr; the error word rides along in slot 7 and is checked
+    void word64_to(const u64* d, int k, u32 count = 1) {
+        slots.src[k] = d;
+        slots.words[k] = 2 * count;
+    }
+    // All slots into hr. The error word rides along in slot 7 and is checked, the trail's
+    // length in slot 6, and the last table's size where it has not been read yet.
+    bool ot_total_due = false;
     void read_slots_checked(u32 stage_err_mask = ~0u) {
         word_to(counters.p + 1, 7);
-        rt.d2h(hr, hslot(0), 8 * sizeof(u64));
+        word_to(counters.p + 0, 6);
+        if (ot_total_due) word_to(ot_off.p + D, 5);
+#if SIGMA_CUDA
+        rt.launches++;
+        rt.syncs++;
+        read_slots_k<<<1, 32, 0, rt.stream>>>(slots, (u64*)rt.pin);
+        ck(cudaGetLastError(), "launch");
+        ck(cudaStreamSynchronize(rt.stream), "sync");
+        std::memcpy(hr, rt.pin, sizeof hr);
+#else
+        for (int k = 0; k < 8; k++) hr[k] = read_slot(slots, k);
+#endif
+        slots = ReadSlots{};
+        ntrail = (u32)hr[6];
+        if (ot_total_due) alg_bytes += 4ull * (u32)hr[5];
+        ot_total_due = false;
         check_err((u32)hr[7] & stage_err_mask);
     }
     u32 read_err() {
@@ -757,10 +788,9 @@ struct pf_sigma_ctx {
         u32 shift = 0, nb = 0;
         if (otb_plan(shift, nb)) {
             create_ot_buckets(shift, nb);
-            word_to(ot_off.p + D, 0);
-            read_slots_checked();
             ot_dirty = false;
-            alg_bytes += 2ull * (4ull * nlits_used + 8ull * ncls) + 8ull * D + 4ull * (u32)hr[0];
+            ot_total_due = true;
+            alg_bytes += 2ull * (4ull * nlits_used + 8ull * ncls) + 8ull * D;
             return;
         }
 #endif
@@ -775,11 +805,9 @@ struct pf_sigma_ctx {
         rt.d2d(ot_cursor.p, ot_off.p, (size_t)D * 4);
         c = view();
         rt.each(FScatter{c}, ncls);
-        word_to(ot_off.p + D, 0);
-        read_slots_checked();
-        const u32 total = (u32)hr[0];
         ot_dirty = false;
-        alg_bytes += 2ull * (4ull * nlits_used + 8ull * ncls) + 8ull * D + 4ull * total;
+        ot_total_due = true;
+        alg_bytes += 2ull * (4ull * nlits_used + 8ull * ncls) + 8ull * D;
     }
 
     // The mean occurrence-list length (literals in use per literal slot) times the
@@ -881,13 +909,11 @@ struct pf_sigma_ctx {
                                            rt.stream),
                "cooperative launch");
             word_to(counters.p + 26, 0);
-            word_to(counters.p + 0, 1);
             read_slots_checked();
             const u32 waves = (u32)hr[0];
             if (trace_on) print_prop_trace(waves);
             wave_stamp += waves + 1;
             prop_waves += waves;
-            ntrail = (u32)hr[1];
             prop_head = ntrail;
         }
 #else
@@ -955,7 +981,7 @@ struct pf_sigma_ctx {
         a.f_npvs = nf ? f_npvs.p : nullptr;
         const u32 nform = nf ? nf : 1u;
         rt.zero(score.p, (size_t)(nvars + 1) * 4);
-        write_u32(counters.p + 27, 0);
+        rt.zero(counters.p + 27, 4);
         rt.each(FScores{a, counters.p + 27}, nvars + 1);
         // LCV order: stable by score over ascending variables (rSort, sort.h:123-133);
         // radix passes only over the bytes the largest score uses
@@ -1091,8 +1117,37 @@ struct pf_sigma_ctx {
         rt.each_dyn(Perm<F>{f, pv_perm.p + perm_off}, perm_n, counters.p + 11);
     }
 
-    // working set of the elected lists, accumulated by the sort kernel
-    u64 pv_bytes() { return read_slots(ws_slots.p); }
+    // What the stages after the sort need of the elected variables, read together: the
+    // working set of their lists (summed by the sort kernel) and, when they are to be
+    // eliminated, whether SUB can derive a unit and the words of BVE scratch (the lists
+    // only get shorter until BVE). n: elected variables of the elimination.
+    bool sub_units_possible = false;
+    u64 ve_scr_words = 0;
+    bool sub_on() const { return opt.sub || opt.ve_plus; }
+    void pv_prepare(u32 n) {
+        word64_to(ws_slots.p, 1, kSpreadSlots);
+        if (n && sub_on()) {
+            SubArgs a{};
+            a.c = view();
+            a.pvs = pvs.p;
+            a.npvs = n;
+            a.sub_max = (u32)opt.sub_max;
+            rt.zero(counters.p + 5, 4);
+            fx_prod.reserve(rt, n + 1);
+            rt.each(FSubPossible{a, counters.p + 5, fx_prod.p}, n);
+            word_to(counters.p + 5, 2);
+        }
+        if (n && opt.ve) {
+            ve_scr_off.reserve(rt, n + 1);
+            big64a.reserve(rt, n + 1);
+            rt.each(FBveNeed{view(), pvs.p, big64a.p}, n);
+            scan_to(big64a.p, ve_scr_off.p, n, 0);
+        }
+        read_slots_checked();
+        ve_scr_words = hr[0];
+        phase_ws = hr[1];
+        sub_units_possible = hr[2] != 0;
+    }
 
     // One SUB pass over the elected variables (warp per variable).
     void sub_pass(const SubArgs& a) {
@@ -1109,7 +1164,7 @@ struct pf_sigma_ctx {
 
     // SUB (elimination.cpp:110-129).
     void sub() {
-        if (!(opt.sub || opt.ve_plus) || !npvs) return;
+        if (!sub_on() || !npvs) return;
         proof_reserve(phase_ws / 2 + 16);  // at most two lines per clause of the elected lists
         SubArgs a;
         a.c = view();
@@ -1122,11 +1177,8 @@ struct pf_sigma_ctx {
         a.pre_off = nullptr;
         a.pre_lits = nullptr;
         a.run = nullptr;
-        write_u32(counters.p + 5, 0);
-        fx_prod.reserve(rt, npvs + 1);
-        rt.each(FSubPossible{a, counters.p + 5, fx_prod.p}, npvs);
         kbytes[K_SUB] += phase_ws;
-        if (read_u32(counters.p + 5) == 0) {
+        if (!sub_units_possible) {
             kclock[K_SUB].start(rt);
             sub_pass(a);
             kclock[K_SUB].stop(rt);
@@ -1320,15 +1372,9 @@ struct pf_sigma_ctx {
         ve_nwit.reserve(rt, npvs);
         ve_def.reserve(rt, npvs);
         ve_cls_scan.reserve(rt, npvs);
-        ve_scr_off.reserve(rt, npvs + 1);
         ve_lit_scan.reserve(rt, npvs);
         ve_wit_scan.reserve(rt, npvs);
-        big64a.reserve(rt, npvs + 1);
-        rt.each(FBveNeed{c, pvs.p, big64a.p}, npvs);
-        scan_to(big64a.p, ve_scr_off.p, npvs, 0);
-        read_slots_checked();
-        const u64 scr_words = hr[0];
-        ve_scr.reserve(rt, (size_t)scr_words + 16);
+        ve_scr.reserve(rt, (size_t)ve_scr_words + 16);
         BveArgs a;
         a.c = c;
         a.pvs = pvs.p;
@@ -1405,9 +1451,9 @@ struct pf_sigma_ctx {
         nlits_used += add_lits;
         proof_clauses(first_new);
         nresolved += add_wit;
-        word_to(counters.p + 0, 0);
-        read_slots_checked();
-        ntrail = (u32)hr[0];
+        // the units and the error word are read with the next stage's values (BCE and the
+        // counts) unless stage dumps are being recorded
+        if (opt.dump_level) read_slots_checked();
         alg_bytes += 4ull * add_lits + 8ull * add_cls + 4ull * add_wit;
     }
 
@@ -1522,14 +1568,18 @@ struct pf_sigma_ctx {
 #else
         rt.each(FCount{a}, ncls);
 #endif
-        rt.d2d(hslot(0), counters64.p + 2, 16);
+        word64_to(counters64.p + 2, 0);
+        word64_to(counters64.p + 3, 1);
         read_slots_checked();
         n_cls_after = (i64)hr[0];
         n_lits_after = (i64)hr[1];
     }
 
-    // shrinkSimp (simplify.cpp:234-245).
-    void gc() {
+    // shrinkSimp (simplify.cpp:234-245). counted: no clause has changed since the last
+    // count, so the sizes that are kept are known.
+    void gc() { compact_store(false); }
+    void gc_counted() { compact_store(true); }
+    void compact_store(bool counted) {
         if (!ncls) {
             compact = true;
             return;
@@ -1542,9 +1592,15 @@ struct pf_sigma_ctx {
         rt.each(FGcFlags{c, big32a.p, big64a.p}, ncls);
         scan_to(big32a.p, big32b.p, ncls, 0);
         scan_to(big64a.p, big64b.p, ncls, 1);
-        read_slots_checked();
-        const u32 keep = (u32)hr[0];
-        const u64 keep_lits = hr[1];
+        u32 keep = (u32)n_cls_after;
+        u64 keep_lits = (u64)n_lits_after;
+        if (counted) {
+            slots = ReadSlots{};
+        } else {
+            read_slots_checked();
+            keep = (u32)hr[0];
+            keep_lits = hr[1];
+        }
         hdr2.reserve(rt, hdr.n);
         cstamp2.reserve(rt, hdr.n);
         lits2.reserve(rt, std::max<size_t>(lits.n, (size_t)keep_lits + 16));
@@ -1569,7 +1625,7 @@ struct pf_sigma_ctx {
         const int times = phase + 1;
         const bool sched = opt.gc_freq > 0 && times > 1 && times != opt.phases && (times % opt.gc_freq) == 0;
         const bool sparse = opt.dump_level == 0 && ncls >= kSparseGcMin && (u64)n_cls_after * 4 < ncls;
-        if (sched || sparse) gc();
+        if (sched || sparse) gc_counted();
     }
     static constexpr u32 kSparseGcMin = 1u << 20;
 
@@ -1581,32 +1637,25 @@ struct pf_sigma_ctx {
     // Per-phase figures of the round (pf_round_stats phase_*): opened at the top of
     // a phase with the live counts entering it, closed where the phase ends.
     u64 ph_bytes0 = 0;
-    double ph_ms0 = 0;
-    double stage_ms_sum() const {
-        double t = 0;
-        for (double x : st.ms_stage) t += x;
-        return t;
-    }
+    int ph_open = -1;  // the phase that the stage times go to (-1: none)
     void phase_open(i64 cls, i64 lits) {
         if (phase >= 8) return;
         st.phase_clauses[phase] = (u64)cls;
         st.phase_literals[phase] = (u64)lits;
         ph_bytes0 = alg_bytes;
-        ph_ms0 = stage_ms_sum();
+        ph_open = phase;
     }
     void phase_close() {
         if (phase >= 8) return;
         st.phase_elected[phase] = npvs;
         st.phase_bytes[phase] = alg_bytes - ph_bytes0;
-        st.phase_ms[phase] = stage_ms_sum() - ph_ms0;
+        ph_open = -1;
     }
 
-    double timed(int stage, void (pf_sigma_ctx::*fn)()) {
+    void timed(int stage, void (pf_sigma_ctx::*fn)()) {
         tm.start(rt);
         (this->*fn)();
-        const double ms = tm.stop(rt);
-        st.ms_stage[stage] += ms;
-        return ms;
+        tm.stop(rt, stage, ph_open);
     }
 
     // Units of the input (one-literal clauses) before the first phase: the
@@ -1643,15 +1692,15 @@ struct pf_sigma_ctx {
             }
             tm.start(rt);
             const bool go = lcve();
-            st.ms_stage[ST_LCVE] += tm.stop(rt);
+            tm.stop(rt, ST_LCVE, ph_open);
             if (!go) {
                 phase_close();
                 break;
             }
             timed(ST_SORT, &pf_sigma_ctx::sort_ot);
             if (opt.dump_level >= 2) dump_pvlists(phase);
-            const u64 W = pv_bytes();
-            phase_ws = W;
+            pv_prepare(stop(diff) ? 0u : npvs);
+            const u64 W = phase_ws;
             alg_bytes += 2ull * W;  // sort reads and writes the lists (8*occ) ~ bounded by W
             if (stop(diff)) {
                 timed(ST_ERE, &pf_sigma_ctx::ere);
@@ -1681,7 +1730,7 @@ struct pf_sigma_ctx {
         }
         timed(ST_PROP, &pf_sigma_ctx::prop);
         timed(ST_COUNT, &pf_sigma_ctx::count_all);
-        timed(ST_GC, &pf_sigma_ctx::gc);
+        timed(ST_GC, &pf_sigma_ctx::gc_counted);
         st.phases_run = phase;
     }
 
@@ -1708,7 +1757,7 @@ struct pf_sigma_ctx {
         rt.launches += 3 * (bits / 8);
         big64a.reserve(rt, (size_t)n + 1);
         big64b.reserve(rt, (size_t)n + 1);
-        DBuf<uint8_t> lrn;
+        DBuf<uint8_t>& lrn = down_learnt;
         lrn.reserve(rt, n);
         rt.each(FClauseSize{c, big32b.p, big64a.p, lrn.p}, n);
         const u64 total = scan64(big64a.p, big64b.p, n);
@@ -1718,7 +1767,6 @@ struct pf_sigma_ctx {
         if (h_lits) rt.d2h(h_lits, lits2.p, (size_t)total * 4);
         if (h_off) rt.d2h(h_off, big64b.p, ((size_t)n + 1) * 8);
         if (h_learnt) rt.d2h(h_learnt, lrn.p, n);
-        lrn.free();
     }
 
     int fid_bits() const {
@@ -1735,8 +1783,9 @@ struct pf_sigma_ctx {
         if (!W) return;
         if (W >= 0xFFFFFFF0ull) throw std::runtime_error("witness stack too large for 32-bit positions");
         const u32 w = (u32)W;
-        DBuf<u32> flag, scan, rstart, key, val, k2, v2, out;
-        DBuf<u64> words, size, off, fw;
+        DBuf<u32>&flag = rs_flag, &scan = rs_scan, &rstart = rs_start, &key = rs_key, &val = rs_val, &k2 = rs_k2;
+        DBuf<u32>&v2 = rs_v2, &out = rs_out;
+        DBuf<u64>&words = rs_words, &size = rs_size, &off = rs_off, &fw = rs_fsum;
         flag.reserve(rt, w);
         scan.reserve(rt, w);
         rt.each(FRecStart{res_mark.p, flag.p}, w);
@@ -1774,8 +1823,8 @@ struct pf_sigma_ctx {
     // receives the model of the original one(s). A batch's formulas are walked side
     // by side, one warp each.
     void extend(uint8_t* h_values) {
-        DBuf<uint8_t> val, packed;
-        DBuf<u64> pfirst;
+        DBuf<uint8_t>&val = rs_value, &packed = rs_packed;
+        DBuf<u64>& pfirst = rs_pfirst;
         val.reserve(rt, (size_t)nvars + 1);
         ExtendMap m{nullptr, nf ? f_var.p : nullptr, nf};
         u64 npacked = 0;
@@ -1802,8 +1851,9 @@ struct pf_sigma_ctx {
         a.value = val.p;
         a.nres = nresolved;
         a.err = counters.p + 1;
-        DBuf<u32> flag, scan, rstart, key, ord, k2, v2, ffirst;
-        DBuf<u64> words;
+        DBuf<u32>&flag = rs_flag, &scan = rs_scan, &rstart = rs_start, &key = rs_key, &ord = rs_val, &k2 = rs_k2;
+        DBuf<u32>&v2 = rs_v2, &ffirst = rs_first;
+        DBuf<u64>& words = rs_words;
         if (!nf) {
             if (nresolved) {
 #if SIGMA_CUDA
@@ -1863,8 +1913,8 @@ struct pf_sigma_ctx {
         f_units_out.assign(nf, 0);
         const u32 n = ntrail;
         if (!n) return;
-        DBuf<u32> key, val, k2, v2, out;
-        DBuf<u64> fu;
+        DBuf<u32>&key = rs_key, &val = rs_val, &k2 = rs_k2, &v2 = rs_v2, &out = rs_out;
+        DBuf<u64>& fu = rs_fsum;
         key.reserve(rt, n);
         val.reserve(rt, n);
         fu.reserve(rt, nf);
@@ -1945,7 +1995,11 @@ struct pf_sigma_ctx {
 
     // Orders the elected list as [formulas that go on | formulas that stop this
     // phase]; elected variables of dropped formulas leave it. group: per formula.
-    void partition_pvs(const std::vector<u32>& group) {
+    // elected: elected variables per formula; when all of them go on, the list stays.
+    void partition_pvs(const std::vector<u32>& group, const std::vector<u32>& elected) {
+        bool all_go = true;
+        for (u32 f = 0; f < nf; f++) all_go &= group[f] == 1u || elected[f] == 0;
+        if (all_go) return;
         rt.h2d(f_group.p, group.data(), (size_t)nf * 4);
         big32a.reserve(rt, (size_t)npvs + 1);
         big32b.reserve(rt, (size_t)npvs + 1);
@@ -2004,15 +2058,15 @@ struct pf_sigma_ctx {
                     going++;
                 }
             }
-            partition_pvs(group);
-            st.ms_stage[ST_LCVE] += tm.stop(rt);
+            partition_pvs(group, fn);
+            tm.stop(rt, ST_LCVE, ph_open);
             if (!going) {
                 phase_close();
                 continue;
             }
             timed(ST_SORT, &pf_sigma_ctx::sort_ot);
-            const u64 W = pv_bytes();
-            phase_ws = W;
+            pv_prepare(n_go);
+            const u64 W = phase_ws;
             alg_bytes += 2ull * W;
             const u32 all = npvs;
             if (n_go < all) {  // stop(diff): ERE, then leave the loop
@@ -2054,7 +2108,7 @@ struct pf_sigma_ctx {
         timed(ST_PROP, &pf_sigma_ctx::prop);
         timed(ST_COUNT, &pf_sigma_ctx::count_formulas);
         mark_unsat(done);
-        timed(ST_GC, &pf_sigma_ctx::gc);
+        timed(ST_GC, &pf_sigma_ctx::gc_counted);
         st.phases_run = phase;
     }
 };
@@ -2111,7 +2165,7 @@ pf_status pf_sigma_create(const pf_options* opts, pf_sigma_ctx** out) {
             return fail("xormaxarity must be in [2, 20]", PF_EINVAL);
         }
         c->rt.init();
-        c->tm.init();
+        c->rt.init_pin();
         c->counters.reserve(c->rt, 32);
         c->counters64.reserve(c->rt, 8);
         c->rt.zero(c->counters.p, 32 * 4);
@@ -2247,7 +2301,7 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
                 at += len;
             }
             c.write_u64(doff.p + num_clauses, at);
-            DBuf<u64> dfirst, dbase, dcb;
+            DBuf<u64>&dfirst = c.up_first, &dbase = c.up_base, &dcb = c.up_cls;
             dfirst.reserve(rt, batch->nf);
             dbase.reserve(rt, batch->nf);
             dcb.reserve(rt, batch->nf + 1);
@@ -2255,7 +2309,7 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
             rt.h2d(dbase.p, base.data(), batch->nf * 8);
             rt.h2d(dcb.p, batch->clause_begin, (batch->nf + 1) * 8);
             if (num_clauses) rt.each(FRebase{doff.p, dcb.p, dfirst.p, dbase.p, batch->nf}, (u32)num_clauses);
-            rt.sync();
+            rt.sync();  // the host arrays of this block are done with
             off_ptr = doff.p;
         } else if (device) {
             rt.d2d(c.lits.p, lits + off0, L * 4);
@@ -2276,8 +2330,8 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
             else std::memcpy(h.data(), learnt, num_clauses);
             for (u64 i = 0; i < num_clauses; i++) if (h[i]) { c.has_learnt = true; break; }
         }
-        DBuf<u64> dcls;
-        DBuf<u32> dnv;
+        DBuf<u64>& dcls = c.up_cls;
+        DBuf<u32>& dnv = c.up_nv;
         UploadArgs a{c.view(), off_ptr, learnt_ptr, off0, L, 0u, nullptr, nullptr, nullptr};
         if (batch) {
             const u32 nf = batch->nf;
@@ -2305,15 +2359,13 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
             a = UploadArgs{c.view(), off_ptr, learnt_ptr, parts ? 0ull : off0, L, nf, dcls.p, c.f_var.p, dnv.p};
         }
         rt.each(FUpload{a}, (u32)num_clauses);
-        rt.sync();
-        dcls.free();
-        dnv.free();
-        const u32 e = c.read_err();
-        if (e & ERR_INPUT) {
+        u32 state[2];  // trail length (units of one-literal clauses), error word
+        rt.d2h(state, c.counters.p, 8);
+        if (state[1] & ERR_INPUT) {
             c.uploaded = false;
             return fail("invalid clause (empty, literal out of range or repeated variable)", PF_EINVAL);
         }
-        c.ntrail = c.read_u32(c.counters.p + 0);  // units of one-literal clauses
+        c.ntrail = state[0];
         c.uploaded = true;
         c.rounds_run = 0;
         c.compact = false;
@@ -2400,6 +2452,10 @@ pf_status pf_sigma_round(pf_sigma_ctx* ctx, pf_round_stats* stats) {
         c.kclock[k].reset();
         c.kbytes[k] = 0;
     }
+    c.tm.reset();
+    c.whole.reset();
+    c.ph_open = -1;
+    c.ot_total_due = false;
     pf_status status = PF_OK;
     try {
         c.keep_at.reserve(c.rt, (size_t)c.nvars + 1);
@@ -2412,9 +2468,7 @@ pf_status pf_sigma_round(pf_sigma_ctx* ctx, pf_round_stats* stats) {
             c.dump_cnf(0, 0);
             c.dump_trail(0, 0);
         }
-        StageTimer whole;
-        whole.init();
-        whole.start(c.rt);
+        c.whole.start(c.rt);
         if (c.nf) {
             if (c.opt.dump_level > 0) throw std::runtime_error("round dumps are not written for formula batches");
             if (c.opt.proof) throw std::runtime_error("proofs are recorded for single formulas only");
@@ -2422,8 +2476,7 @@ pf_status pf_sigma_round(pf_sigma_ctx* ctx, pf_round_stats* stats) {
         } else if (!(!o.phases && !(o.all || o.ere))) {
             c.round();
         }
-        c.st.ms_total = whole.stop(c.rt);
-        whole.destroy();
+        c.whole.stop(c.rt, 0, 0);
         if (c.opt.dump_level > 0) {
             c.dump_cnf(c.phase, 8);
             c.dump_trail(c.phase, 8);
@@ -2453,8 +2506,13 @@ pf_status pf_sigma_round(pf_sigma_ctx* ctx, pf_round_stats* stats) {
     c.st.host_syncs = c.rt.syncs;
     if (status == PF_OK || status == PF_UNSAT) {
         try {
-            c.rt.sync();
             c.kbytes[pf_sigma_ctx::K_MIS] = c.read_slots(c.ws_slots.p + kSpreadSlots);
+            c.whole.each([&](const StageClock::Span&, double ms) { c.st.ms_total = ms; });
+            c.tm.each([&](const StageClock::Span& s, double ms) {
+                c.st.ms_stage[s.stage] += ms;
+                if (s.phase >= 0) c.st.phase_ms[s.phase] += ms;
+            });
+            c.st.host_syncs = c.rt.syncs;
             for (int k = 0; k < pf_sigma_ctx::K_COUNT; k++) {
                 c.st.ms_kernel[k] = c.kclock[k].total_ms();
                 c.st.bytes_kernel[k] = c.kbytes[k];
@@ -2787,68 +2845,12 @@ pf_status pf_sigma_footprint(pf_sigma_ctx* ctx, uint64_t* bytes) {
 
 void pf_sigma_destroy(pf_sigma_ctx* ctx) {
     if (!ctx) return;
-    // DBuf members release themselves through the runtime
     pf_sigma_ctx& c = *ctx;
-    DBuf<Hdr>* hb[] = {&c.hdr, &c.hdr2, &c.sub_hdrs};
-    for (auto* b : hb) b->free();
-    DBuf<u32>* b32[] = {&c.lits, &c.lits2, &c.ot_off, &c.ot_size, &c.ot_refs, &c.ot_cursor, &c.asg, &c.ps, &c.ns,
-                        &c.pvrank, &c.trail, &c.resolved, &c.counters, &c.score, &c.order, &c.order_k2,
-                        &c.order_v2, &c.rank, &c.bound, &c.pvs, &c.flags, &c.flags_scan, &c.work, &c.cl_stamp,
-                        &c.radix_hist, &c.radix_hscan, &c.scan_tmp32, &c.big32a, &c.big32b, &c.ve_porgs,
-                        &c.ve_norgs, &c.ve_ncls, &c.ve_nlits, &c.ve_nwit, &c.ve_def, &c.ve_cls_scan, &c.ve_scr,
-                        &c.sub_ent, &c.sub_ent_off, &c.sub_ids, &c.sub_words, &c.sub_sizes, &c.sub_pre_off,
-                        &c.sub_pre_lits, &c.sub_ulits, &c.ere_target, &c.ere_losers, &c.cstamp, &c.cstamp2,
-                        &c.keep_at, &c.keep_shape};
-    for (auto* b : b32) b->free();
-    DBuf<u64>* b64[] = {&c.counters64, &c.ws_slots, &c.hread, &c.scan_tmp64, &c.big64a, &c.big64b, &c.ve_scr_off, &c.ve_lit_scan,
-                        &c.ve_wit_scan, &c.sub_wrd, &c.sub_wrd_off, &c.ere_claim, &c.ere_key};
-    for (auto* b : b64) b->free();
-    DBuf<uint8_t>* b8[] = {&c.vstate, &c.ve_type, &c.sub_run};
-    c.mis_word.free();
-    c.mis_resume.free();
-    c.mis_cmin.free();
-#if !SIGMA_CUDA
-    for (auto& b : c.mis_in) b.free();
-#endif
-    c.mis_rec.free();
-    c.mis_gbits.free();
-    c.down_learnt.free();
-    c.up_off.free();
-    c.up_learnt.free();
-    c.res_mark.free();
-#if SIGMA_CUDA
-    c.scan1_agg.free();
-    c.scan1_incl.free();
-    c.scan1_total.free();
-    c.scan1_flag.free();
-    c.scan1_ctl.free();
-#endif
-    c.mis_big_a.free();
-    c.mis_big_b.free();
-#if SIGMA_CUDA
-    c.otb_count.free();
-    c.otb_base.free();
-    c.otb_cursor.free();
-    c.otb_pair.free();
-    c.prop_trace.free();
-    c.prop_parts.free();
-#endif
-    c.pv_perm.free();
-    c.pv_key.free();
-    for (auto* b : b8) b->free();
-    c.sub_units.free();
-    c.sub_units2.free();
-    c.sub_pairs.free();
-    DBuf<u32>* fx[] = {&c.fx_prod, &c.fx_rank, &c.fx_lit, &c.fx_k2, &c.fx_v2, &c.fx_flag, &c.fx_scan, &c.want_rank,
-                       &c.want_lit, &c.want_cnt, &c.want_off, &c.used_lit, &c.used_off};
-    for (auto* b : fx) b->free();
-    c.fx_prod8.free();
-    c.fx_other8.free();
-    c.proof.free();
     c.tm.destroy();
+    c.whole.destroy();
     for (auto& k : c.kclock) k.destroy();
     c.rt.destroy();
-    delete ctx;
+    delete ctx;  // the buffers release themselves through the runtime
 }
 
 const char* pf_last_error(void) { return g_last_error.c_str(); }
