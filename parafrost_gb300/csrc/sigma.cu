@@ -349,8 +349,11 @@ struct pf_sigma_ctx {
     DBuf<u32> mis_gbits;  // the election's graph membership bitmap
     DBuf<u32> pv_perm, pv_key;
     DBuf<u32> work, cl_stamp;
-    DBuf<u32> radix_hist, radix_hscan, scan_tmp32;
+    DBuf<u64> radix_work;
+#if !SIGMA_CUDA
+    DBuf<u32> scan_tmp32;
     DBuf<u64> scan_tmp64;
+#endif
     DBuf<u64> big64a, big64b;
     DBuf<uint8_t> down_learnt;  // learnt flags of the downloaded clauses
     DBuf<u64> up_off;           // offsets of an upload from host buffers
@@ -614,6 +617,16 @@ struct pf_sigma_ctx {
         return read_u64(total);
     }
 #endif
+
+    // Stable radix sort of n (key, value) pairs by the keys' low `bits` bits; the sorted
+    // pairs end in (keys, vals).
+    void sort_pairs(u32* keys, u32* vals, u32* k2, u32* v2, size_t n, int bits) {
+        radix_work.reserve(rt, radix_work_elems(n));
+        if (radix_sort_any(keys, vals, k2, v2, n, bits, radix_work.p, counters.p + 1, rt.stream, rt.launches)) {
+            rt.d2d(keys, k2, n * 4);
+            rt.d2d(vals, v2, n * 4);
+        }
+    }
 
     // ------------------------------------------------------------ dumps
     void rec(u32 kind, u32 ph, u32 stage, const std::vector<u32>& d) {
@@ -989,9 +1002,7 @@ struct pf_sigma_ctx {
         int bits = 8;
         while (bits < 32 && (max_score >> bits)) bits += 8;
         rt.d2d(order_k2.p, score.p + 1, (size_t)nvars * 4);  // keys = score[1..]
-        radix_sort_pairs(order_k2.p, order.p, order_v2.p, rank.p, nvars, bits, radix_hist.p, radix_hscan.p,
-                         scan_tmp32.p, rt.stream);
-        rt.launches += 5 * (bits / 8);
+        sort_pairs(order_k2.p, order.p, order_v2.p, rank.p, nvars, bits);
         rt.zero(bound.p, (size_t)nform * 8, 0xFF);
         rt.each(FRank{a}, nvars);
         // Independent set by rounds. Undecided lists: flags|mis_big_a and
@@ -1106,9 +1117,7 @@ struct pf_sigma_ctx {
         pv_perm.reserve(rt, nvars + 1);
         pv_key.reserve(rt, nvars + 1);
         rt.each(FPvKey{view(), pvs.p, pv_key.p, pv_perm.p, n_go}, npvs);
-        radix_sort_pairs(pv_key.p, pv_perm.p, order_k2.p, order_v2.p, npvs, 8, radix_hist.p, radix_hscan.p,
-                         scan_tmp32.p, rt.stream);
-        rt.launches += 5;
+        sort_pairs(pv_key.p, pv_perm.p, order_k2.p, order_v2.p, npvs, 8);
     }
 
     // f(k) for every elected variable, in work order, dynamically scheduled.
@@ -1224,16 +1233,10 @@ struct pf_sigma_ctx {
                 fx_flag.reserve(rt, (size_t)np + 1);
                 fx_scan.reserve(rt, (size_t)np + 1);
                 rt.each(FSubfxPairLit{sub_pairs.p, sub_units.p, fx_rank.p, fx_lit.p}, np);
-                radix_hist.reserve(rt, radix_hist_elems(np));
-                radix_hscan.reserve(rt, radix_hist_elems(np));
-                scan_tmp32.reserve(rt, scan_tmp_elems(radix_hist_elems(np)) + 4);
                 // by literal, then stable by rank: (rank, literal) order
                 const int lb = key_bits(D), rb = key_bits(npvs);
-                radix_sort_pairs(fx_lit.p, fx_rank.p, fx_k2.p, fx_v2.p, np, lb, radix_hist.p, radix_hscan.p,
-                                 scan_tmp32.p, rt.stream);
-                radix_sort_pairs(fx_rank.p, fx_lit.p, fx_k2.p, fx_v2.p, np, rb, radix_hist.p, radix_hscan.p,
-                                 scan_tmp32.p, rt.stream);
-                rt.launches += 5 * (lb / 8 + rb / 8);
+                sort_pairs(fx_lit.p, fx_rank.p, fx_k2.p, fx_v2.p, np, lb);
+                sort_pairs(fx_rank.p, fx_lit.p, fx_k2.p, fx_v2.p, np, rb);
                 rt.each(FSubfxFirst{fx_rank.p, fx_lit.p, fx_flag.p}, np);
                 nwant = scan32(fx_flag.p, fx_scan.p, np);
                 want_rank.reserve(rt, (size_t)nwant + 1);
@@ -1539,17 +1542,11 @@ struct pf_sigma_ctx {
             big32b.reserve(rt, (size_t)nl + 1);
             work.reserve(rt, 2 * (size_t)nl + 2);
             big64b.reserve(rt, (size_t)nl + 1);
-            radix_hist.reserve(rt, radix_hist_elems(nl));
-            radix_hscan.reserve(rt, radix_hist_elems(nl));
-            scan_tmp32.reserve(rt, scan_tmp_elems(radix_hist_elems(nl)) + 4);
             rt.each(FEreLoserKey{ere_key.p, ere_losers.p, big32b.p, big32a.p, false}, nl);
-            radix_sort_pairs(big32a.p, big32b.p, work.p, work.p + nl + 1, nl, 32, radix_hist.p, radix_hscan.p,
-                             scan_tmp32.p, rt.stream);
+            sort_pairs(big32a.p, big32b.p, work.p, work.p + nl + 1, nl, 32);
             rt.each(FEreLoserKey{ere_key.p, ere_losers.p, big32b.p, big32a.p, true}, nl);
             const int rb = key_bits(npvs);
-            radix_sort_pairs(big32a.p, big32b.p, work.p, work.p + nl + 1, nl, rb, radix_hist.p, radix_hscan.p,
-                             scan_tmp32.p, rt.stream);
-            rt.launches += 5 * (4 + rb / 8);
+            sort_pairs(big32a.p, big32b.p, work.p, work.p + nl + 1, nl, rb);
             rt.each(FEreLoserGather{ere_key.p, ere_losers.p, big32b.p, big64b.p}, nl);
             rt.one(FEreFix{a, big64b.p, nl});
         }
@@ -1745,16 +1742,11 @@ struct pf_sigma_ctx {
         big32a.reserve(rt, (size_t)n + 1);
         big32b.reserve(rt, (size_t)n + 1);
         work.reserve(rt, 2 * (size_t)n + 2);
-        radix_hist.reserve(rt, radix_hist_elems(n));
-        radix_hscan.reserve(rt, radix_hist_elems(n));
-        scan_tmp32.reserve(rt, scan_tmp_elems(radix_hist_elems(n)) + 4);
         const Ctx c = view();
         rt.each(FClauseFid{c, big32a.p, big32b.p}, n);
         int bits = 8;
         while (bits < 32 && (nf >> bits)) bits += 8;
-        radix_sort_pairs(big32a.p, big32b.p, work.p, work.p + n + 1, n, bits, radix_hist.p, radix_hscan.p,
-                         scan_tmp32.p, rt.stream);
-        rt.launches += 3 * (bits / 8);
+        sort_pairs(big32a.p, big32b.p, work.p, work.p + n + 1, n, bits);
         big64a.reserve(rt, (size_t)n + 1);
         big64b.reserve(rt, (size_t)n + 1);
         DBuf<uint8_t>& lrn = down_learnt;
@@ -1803,12 +1795,8 @@ struct pf_sigma_ctx {
         if (!h_out) return;
         k2.reserve(rt, R + 1);
         v2.reserve(rt, R + 1);
-        radix_hist.reserve(rt, radix_hist_elems(R));
-        radix_hscan.reserve(rt, radix_hist_elems(R));
-        scan_tmp32.reserve(rt, scan_tmp_elems(radix_hist_elems(R)) + 4);
         const int bits = fid_bits();
-        radix_sort_pairs(key.p, val.p, k2.p, v2.p, R, bits, radix_hist.p, radix_hscan.p, scan_tmp32.p, rt.stream);
-        rt.launches += 5 * (bits / 8);
+        sort_pairs(key.p, val.p, k2.p, v2.p, R, bits);
         size.reserve(rt, R + 1);
         off.reserve(rt, R + 1);
         rt.each(FRecSize{words.p, val.p, size.p}, R);
@@ -1879,12 +1867,8 @@ struct pf_sigma_ctx {
             rt.each(FRecFid{c, rstart.p, R, w, key.p, ord.p, words.p, nullptr}, R);
             k2.reserve(rt, R + 1);
             v2.reserve(rt, R + 1);
-            radix_hist.reserve(rt, radix_hist_elems(R));
-            radix_hscan.reserve(rt, radix_hist_elems(R));
-            scan_tmp32.reserve(rt, scan_tmp_elems(radix_hist_elems(R)) + 4);
             const int bits = fid_bits();
-            radix_sort_pairs(key.p, ord.p, k2.p, v2.p, R, bits, radix_hist.p, radix_hscan.p, scan_tmp32.p, rt.stream);
-            rt.launches += 5 * (bits / 8);
+            sort_pairs(key.p, ord.p, k2.p, v2.p, R, bits);
             ffirst.reserve(rt, nf + 1);
             rt.each(FExtendFirst{key.p, R, ffirst.p}, nf + 1);
             a.rec_start = rstart.p;
@@ -1925,12 +1909,8 @@ struct pf_sigma_ctx {
         if (!h_out) return;
         k2.reserve(rt, n);
         v2.reserve(rt, n);
-        radix_hist.reserve(rt, radix_hist_elems(n));
-        radix_hscan.reserve(rt, radix_hist_elems(n));
-        scan_tmp32.reserve(rt, scan_tmp_elems(radix_hist_elems(n)) + 4);
         const int bits = fid_bits();
-        radix_sort_pairs(key.p, val.p, k2.p, v2.p, n, bits, radix_hist.p, radix_hscan.p, scan_tmp32.p, rt.stream);
-        rt.launches += 5 * (bits / 8);
+        sort_pairs(key.p, val.p, k2.p, v2.p, n, bits);
         out.reserve(rt, n);
         rt.each(FUnitGather{c, val.p, key.p, f_var.p, out.p}, n);
         rt.d2h(h_out, out.p, (size_t)n * 4);
@@ -2270,9 +2250,6 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
         c.flags_scan.reserve(rt, num_vars + 1);
         c.mis_word.reserve(rt, num_vars + 1);
         c.mis_resume.reserve(rt, num_vars + 1);
-        c.radix_hist.reserve(rt, radix_hist_elems(num_vars + 1));
-        c.radix_hscan.reserve(rt, radix_hist_elems(num_vars + 1));
-        c.scan_tmp32.reserve(rt, scan_tmp_elems(std::max<size_t>(radix_hist_elems(num_vars + 1), cap_cls)) + 4);
         rt.zero(c.asg.p, (size_t)(num_vars + 1) * 4);
         rt.zero(c.vstate.p, num_vars + 1);
         rt.zero(c.counters.p, 32 * 4);
