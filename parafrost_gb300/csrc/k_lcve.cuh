@@ -34,49 +34,80 @@ HD u32 mis_dec_bits(u32 d) { return d << 30; }
 struct LcveArgs {
     Ctx c;
     u32 pt, nt;           // mu_pos << mu_inc, mu_neg << mu_inc
-    u32* score;           // nvars+1
-    u32* order;           // nvars: variables in (score, var) order
-    u32* rank;            // nvars+1
+    u32* score;           // nvars+1 (stage dumps)
+    u32* cand;            // candidates in variable order (lcve_class in the top bits)
+    u32* order;           // the same in (score, variable) order
+    u32 ncand;
+    bool dirty;           // ps/ns hold the occurrences (else the lists' sizes are they)
+    bool all;             // every variable is listed (stage dumps record the whole order)
+    u32* max_score;
+    u32* key;             // the candidates' scores
     u32* word;            // nvars+1: independent-set words
     u32* resume;          // nvars+1: where each vertex's last pull walk stopped
     const Q4* crec;       // per clause: its first three literals and size | deleted << 31
     u64* ws_bytes;        // kSpreadSlots words summing the graph's working set (4*occ + sum(8 + 4*len))
-    u32* gbits;           // graph membership, one bit per variable (zeroed before k_mis_init)
     u32* bound;           // per formula f: [2f] = B0 (first valid non-F rank), [2f+1] = B
     const u32* f_active;  // batches: formulas taking part in this election (null: all)
-    u32* f_npvs;          // batches: elected variables per formula
+    u32* f_npvs;          // batches: elected variables per formula, counted up to lcve_min (at least 1)
+    u32 lcve_min;
+    u32 nform;            // formulas (1 without a batch)
     u32* pvs;             // elected variables in rank order
     u64 pf = 0, pl = 0;   // L2 policies in the rounds kernel: streams go first, words last
     u32* cmin;            // per clause: the least rank of its graph vertices (MIS_NO_RANK when
                           // it has none or is deleted), built with the clause records
 };
 
-// write_scores (histogram.h:32-41): eligible[v-1] = v, scores[v] = ps*ns (32-bit wrap).
-// The largest score goes to max_score (it sets how many radix passes the order needs).
-HD void k_scores(const LcveArgs& a, u32* max_score, u32 v) {
-    u32 sc = 0;
-    if (v) {
-        sc = a.c.ps[v] * a.c.ns[v];
-        a.score[v] = sc;
-        a.order[v - 1] = v;
+// A listed variable carries its class in the two bits above its number (numbers stay
+// below 2^30), so the passes over the candidates read nothing else of it.
+enum : u32 { LC_FIXED = 0, LC_SMALL = 1, LC_BIG = 2, LC_INVALID = 3 };
+constexpr u32 LC_VAR = 0x3FFFFFFFu;
+HD u32 lc_var(u32 x) { return x & LC_VAR; }
+HD u32 lc_class(u32 x) { return x >> 30; }
+
+HD u32 lcve_ps(const LcveArgs& a, u32 v) { return a.dirty ? a.c.ps[v] : a.c.ot_size[V2L(v)]; }
+HD u32 lcve_ns(const LcveArgs& a, u32 v) { return a.dirty ? a.c.ns[v] : a.c.ot_size[NEG(V2L(v))]; }
+
+// The candidates, in variable order: variables that occur, are not eliminated and belong
+// to a formula taking part, with their scores (write_scores, histogram.h:32-41: ps*ns,
+// 32-bit wrap) as sort keys. The others cannot be elected, bound the election or be a
+// neighbour in a live clause, so every later pass of the election runs over the
+// candidates alone: a formula that has shrunk costs what is left of it, not its
+// variable count (elections without their rounds, six phases over 20M variables of a
+// community formula that shrinks to 180 clauses: 13.4 ms over all variables, 7.9 over
+// the candidates; a 6.8M-clause AIG 2.1 and 1.4 ms). The largest score goes to max_score (it sets how many radix passes
+// the order needs). One scan over the variables (value, then put).
+// Class: not freezable (a bound of the election), or freezable with short or long lists.
+constexpr u32 MIS_WARP_MIN_OCC = 32;
+struct LcveCand {
+    LcveArgs a;
+    HD u32 value(size_t i) const {
+        const u32 v = (u32)i + 1u;
+        const u32 p = lcve_ps(a, v), n = lcve_ns(a, v);
+        const bool valid = (p || n) && !a.c.vstate[v] && (!a.f_active || a.f_active[fid_of(a.c, v)]);
+        a.word[v] = MIS_NO_RANK;
+        if (a.all) a.score[v] = p * n;
+        warp_max_atomic(a.max_score, valid || a.all ? p * n : 0u);
+        return valid || a.all;
     }
-    warp_max_atomic(max_score, sc);
-}
+    HD void put(size_t i, u32 take, u32 at) const {
+        if (!take) return;
+        const u32 v = (u32)i + 1u;
+        const u32 p = lcve_ps(a, v), n = lcve_ns(a, v);
+        u32 cl = LC_FIXED;
+        if (a.all && (!(p || n) || a.c.vstate[v])) cl = LC_INVALID;
+        else if (p < a.pt || n < a.nt)
+            cl = a.c.ot_size[V2L(v)] + a.c.ot_size[NEG(V2L(v))] > MIS_WARP_MIN_OCC ? LC_BIG : LC_SMALL;
+        a.key[at] = p * n;
+        a.cand[at] = a.order[at] = v | cl << 30;
+    }
+};
 
-HD bool lcve_valid(const Ctx& c, u32 v) {
-    if (c.vstate[v]) return false;
-    return !(c.ps[v] == 0 && c.ns[v] == 0);
-}
-HD bool lcve_freezable(const LcveArgs& a, u32 v) { return a.c.ps[v] < a.pt || a.c.ns[v] < a.nt; }
-HD bool lcve_big(const LcveArgs& a, u32 v) {
-    return a.c.ot_size[V2L(v)] >= a.pt && a.c.ot_size[NEG(V2L(v))] >= a.nt;
-}
-
-// rank[v] and B0 = first valid candidate outside F.
+// Place p of the order: a freezable variable's word takes its rank; B0 = first valid
+// candidate outside F.
 HD void k_rank(const LcveArgs& a, u32 p) {
-    const u32 v = a.order[p];
-    a.rank[v] = p;
-    if (lcve_valid(a.c, v) && !lcve_freezable(a, v)) atom_min(&a.bound[2 * fid_of(a.c, v)], p);
+    const u32 x = a.order[p], cl = lc_class(x), v = lc_var(x);
+    if (cl == LC_FIXED) atom_min(&a.bound[2 * fid_of(a.c, v)], p);
+    else if (cl != LC_INVALID) a.word[v] = p;
 }
 
 // The independent set is decided in rounds. In a round every undecided vertex walks its
@@ -91,8 +122,6 @@ HD void k_rank(const LcveArgs& a, u32 p) {
 // the clauses a walk has passed never need another look. Vertices with more than
 // MIS_WARP_MIN_OCC clauses are walked by a whole warp; the others by one thread,
 // or by a group of lanes when few of them are left (mis_lanes).
-constexpr u32 MIS_WARP_MIN_OCC = 32;
-
 struct MisFront {
     u32* small;   // list of small-adjacency vertices
     u32* nsmall;
@@ -100,50 +129,47 @@ struct MisFront {
     u32* nbig;
 };
 
-HD bool mis_is_big(const Ctx& c, u32 v) { return c.ot_size[V2L(v)] + c.ot_size[NEG(V2L(v))] > MIS_WARP_MIN_OCC; }
-
-HD void mis_append(const MisFront& f, const Ctx& c, u32 v, bool pred) {
-    const bool big = pred && mis_is_big(c, v);
-    const u32 ps = warp_append(f.nsmall, pred && !big);
-    const u32 pb = warp_append(f.nbig, big);
-    if (pred && !big) f.small[ps] = v;
-    if (big) f.big[pb] = v;
-}
-
-// Graph membership; every graph vertex starts on the undecided lists.
-HD void k_mis_init(const LcveArgs& a, const MisFront& und, u32 v) {
-    const u32 f = v ? fid_of(a.c, v) : 0u;
-    const bool in_graph = v && (!a.f_active || a.f_active[f]) && lcve_valid(a.c, v) && lcve_freezable(a, v) &&
-                          a.rank[v] < a.bound[2 * f];
-    a.word[v] = in_graph ? a.rank[v] : MIS_NO_RANK;
+// Graph membership of candidate i (in variable order, so that the walks of neighbouring
+// vertices read neighbouring lists): freezable and before the first bound. Every graph
+// vertex starts on the undecided lists. The election's bound starts at B0.
+HD bool mis_vertex(const LcveArgs& a, u32 i, u32& v, bool& big) {
+    if (i < a.nform) a.bound[2 * i + 1] = a.bound[2 * i];
+    if (i >= a.ncand) return false;
+    const u32 x = a.cand[i], cl = lc_class(x);
+    v = lc_var(x);
+    big = cl == LC_BIG;
+    if (cl != LC_SMALL && cl != LC_BIG) return false;
+    if (a.word[v] >= a.bound[2 * fid_of(a.c, v)]) {
+        a.word[v] = MIS_NO_RANK;
+        return false;
+    }
     a.resume[v] = 0;
-    bitmap_set(a.gbits, v, in_graph);
-    mis_append(und, a.c, v, in_graph);
+    return true;
 }
 
-#if SIGMA_CUDA
-// k_mis_init over variables 0..n-1 with block-wide appends: a block takes 256
-// consecutive variables a step, ranks its small and big vertices by warp ballots and
+#if !SIGMA_CUDA
+HD void k_mis_init(const LcveArgs& a, const MisFront& und, u32 i) {
+    u32 v = 0;
+    bool big = false;
+    if (!mis_vertex(a, i, v, big)) return;
+    if (big) und.big[atom_add(und.nbig, 1u)] = v;
+    else und.small[atom_add(und.nsmall, 1u)] = v;
+}
+#else
+// k_mis_init over n >= max(ncand, nform) items with block-wide appends: a block takes 256
+// consecutive candidates a step, ranks its small and big vertices by warp ballots and
 // reserves both lists' places with one atomic each (the lists' two counters would
-// otherwise take one atomic per warp step over 20M variables); lane 0 of a warp
-// writes its 32 variables' membership word.
+// otherwise take one atomic per warp step over 20M candidates).
 __global__ void __launch_bounds__(256) mis_init_k(LcveArgs a, MisFront und, u32 n) {
     __shared__ u32 ws[8], wb[8], base_s, base_b;
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (u32 v0 = blockIdx.x * 256u; v0 < n; v0 += gridDim.x * 256u) {
-        const u32 v = v0 + threadIdx.x;
-        bool in_graph = false, big = false;
-        if (v < n) {
-            const u32 f = v ? fid_of(a.c, v) : 0u;
-            in_graph = v && (!a.f_active || a.f_active[f]) && lcve_valid(a.c, v) && lcve_freezable(a, v) &&
-                       a.rank[v] < a.bound[2 * f];
-            a.word[v] = in_graph ? a.rank[v] : MIS_NO_RANK;
-            a.resume[v] = 0;
-            big = in_graph && mis_is_big(a.c, v);
-        }
-        const u32 gm = __ballot_sync(kFull, in_graph);
-        if (lane == 0 && v < n) a.gbits[v >> 5] = gm;
-        const u32 ms = __ballot_sync(kFull, in_graph && !big), mb = __ballot_sync(kFull, big);
+    for (u32 i0 = blockIdx.x * 256u; i0 < n; i0 += gridDim.x * 256u) {
+        u32 v = 0;
+        bool big = false;
+        const bool in = mis_vertex(a, i0 + threadIdx.x, v, big);
+        const bool small = in && !big;
+        big = in && big;
+        const u32 ms = __ballot_sync(kFull, small), mb = __ballot_sync(kFull, big);
         if (lane == 0) {
             ws[warp] = (u32)__popc(ms);
             wb[warp] = (u32)__popc(mb);
@@ -163,7 +189,7 @@ __global__ void __launch_bounds__(256) mis_init_k(LcveArgs a, MisFront und, u32 
         }
         __syncthreads();
         const u32 below = (1u << lane) - 1u;
-        if (in_graph && !big) und.small[base_s + ws[warp] + (u32)__popc(ms & below)] = v;
+        if (small) und.small[base_s + ws[warp] + (u32)__popc(ms & below)] = v;
         if (big) und.big[base_b + wb[warp] + (u32)__popc(mb & below)] = v;
         __syncthreads();
     }
@@ -210,9 +236,9 @@ HD const u32* mis_long_lits(const LcveArgs& a, const MisCl& cl) {
     return cl.size() > 3 ? a.c.lits + hdr_ro(&a.c.hdr[cl.r]).start : nullptr;
 }
 
-// The record of clause i, and the graph's working set: every graph vertex's list
-// entry (4 bytes) and, for a live clause, its header and literals (8 + 4*len) once
-// per graph vertex in it. Runs after k_mis_init.
+// The record of clause i, its least graph rank, and the graph's working set: every graph
+// vertex's list entry (4 bytes) and, for a live clause, its header and literals
+// (8 + 4*len) once per graph vertex in it. Runs after the graph is known.
 HD void k_mis_rec(const LcveArgs& a, Q4* rec, u32 i) {
     const Ctx& c = a.c;
     const Hdr h = c.hdr[i];
@@ -225,9 +251,8 @@ HD void k_mis_rec(const LcveArgs& a, Q4* rec, u32 i) {
     rec[i] = q;
     u32 ng = 0, m = MIS_NO_RANK;
     for (u32 k = 0; k < h.size; k++) {
-        const u32 x = ABS(l[k]);
-        ng += (ldro(&a.gbits[x >> 5]) >> (x & 31u)) & 1u;
-        const u32 rk = mis_rank(a.word[x]);
+        const u32 rk = mis_rank(a.word[ABS(l[k])]);
+        ng += rk != MIS_NO_RANK;
         if (rk < m) m = rk;
     }
     a.cmin[i] = h_deleted(h.flags) ? MIS_NO_RANK : m;
@@ -286,10 +311,10 @@ __global__ void __launch_bounds__(256) mis_rec_warp_k(LcveArgs a, Q4* rec) {
             const u32 st = __shfl_sync(0xffffffffu, start, k & 31u), ex = __shfl_sync(0xffffffffu, excl, k & 31u);
             const u32 wt = __shfl_sync(0xffffffffu, weight, k & 31u);
             if (j < total) {
-                const u32 x = ABS(__ldg(&a.c.lits[st + (j - ex)]));
-                if ((ldro(&a.gbits[x >> 5]) >> (x & 31u)) & 1u) {
+                const u32 rk = mis_rank(ldro(&a.word[ABS(__ldg(&a.c.lits[st + (j - ex)]))]));
+                if (rk != MIS_NO_RANK) {
                     sum += wt;
-                    atomicMin(&s_min[(threadIdx.x & ~31u) + (k & 31u)], mis_rank(ldro(&a.word[x])));
+                    atomicMin(&s_min[(threadIdx.x & ~31u) + (k & 31u)], rk);
                 }
             }
         }
@@ -325,6 +350,13 @@ HD bool mis_blocked_in(const LcveArgs& a, u32 v, u32 rv, const MisCl& cl) {
     return false;
 }
 
+// Vertex v (rank rv) goes in; one whose lists reach the temperatures bounds the election
+// (B = min(B0, first member whose lists reach them)).
+HD void mis_goes_in(const LcveArgs& a, u32 v, u32 rv, u32 np, u32 nn) {
+    atom_or(&a.word[v], mis_dec_bits(MIS_IN));
+    if (np >= a.pt && nn >= a.nt) atom_min(&a.bound[2 * fid_of(a.c, v) + 1], rv);
+}
+
 // Pull walk of undecided vertex v by one thread: true when v went in; otherwise the
 // resume point is stored (v stays undecided). The next clause's record is loaded
 // before the current one is examined.
@@ -345,7 +377,7 @@ HD bool mis_pull_one(const LcveArgs& a, u32 v, u32 wv, bool r0) {
             cl = nx;
         }
     }
-    atom_or(&a.word[v], mis_dec_bits(MIS_IN));
+    mis_goes_in(a, v, rv, np, n - np);
     return true;
 }
 
@@ -391,7 +423,7 @@ HD void k_mis_pull(const LcveArgs& a, const u32* in, const MisFront& und, const 
     const u32 v = in[idx];
     const u32 wv = a.word[v];
     if (mis_dec(wv) != MIS_UNDECIDED) return;
-    const bool big = mis_is_big(a.c, v);
+    const bool big = a.c.ot_size[V2L(v)] + a.c.ot_size[NEG(V2L(v))] > MIS_WARP_MIN_OCC;
     if (mis_pull_one(a, v, wv, r0)) {
         if (big) ins.big[atom_add(ins.nbig, 1u)] = v;
         else ins.small[atom_add(ins.nsmall, 1u)] = v;
@@ -511,7 +543,7 @@ DEV bool mis_try(const LcveArgs& a, u32 v, u32 gm, u32 gbase, u32 sub, u32 L, u3
             return false;
         }
     }
-    if (sub == 0) atomicOr(&a.word[v], mis_dec_bits(MIS_IN));
+    if (sub == 0) mis_goes_in(a, v, rv, np, n - np);
     for (u32 t = sub; t < n; t += L)
         mis_push_clause(a, v, rv, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf), false));
     return true;
@@ -655,29 +687,25 @@ __global__ void __launch_bounds__(256, 6) mis_rounds_k(LcveArgs a0, MisRounds w)
 }
 #endif
 
-// B starts at B0, per formula.
-HD void k_bound_init(const LcveArgs& a, u32 f) { a.bound[2 * f + 1] = a.bound[2 * f]; }
-
-// B = min(B0, first member whose lists reach the temperatures).
-HD void k_mis_bound(const LcveArgs& a, u32 v) {
-    if (v == 0) return;
-    const u32 w = a.word[v];
-    if (mis_rank(w) != MIS_NO_RANK && mis_dec(w) == MIS_IN && lcve_big(a, v)) atom_min(&a.bound[2 * fid_of(a.c, v) + 1], a.rank[v]);
-}
-
-// Election flags over rank positions below B (compacted by the caller in rank order).
-HD void k_elect_flag(const LcveArgs& a, u32* flags, u32 p) {
-    const u32 v = a.order[p];
-    const u32 w = a.word[v];
-    flags[p] = (p < a.bound[2 * fid_of(a.c, v) + 1] && mis_rank(w) != MIS_NO_RANK && mis_dec(w) == MIS_IN) ? 1u : 0u;
-}
-
-HD void k_elect_write(const LcveArgs& a, const u32* flags, const u32* scan, u32 p) {
-    if (!flags[p]) return;
-    const u32 v = a.order[p];
-    a.pvs[scan[p]] = v;
-    a.c.pvrank[v] = scan[p];
-    if (a.f_npvs) atom_add(&a.f_npvs[fid_of(a.c, v)], 1u);
-}
+// The elected variables: the members of the set below their formula's bound, in rank
+// order. One scan over the order.
+struct LcveElect {
+    LcveArgs a;
+    HD u32 value(size_t p) const {
+        const u32 v = lc_var(a.order[p]);
+        const u32 w = a.word[v];
+        return (u32)p < a.bound[2 * fid_of(a.c, v) + 1] && mis_rank(w) != MIS_NO_RANK && mis_dec(w) == MIS_IN;
+    }
+    HD void put(size_t p, u32 take, u32 at) const {
+        if (!take) return;
+        const u32 v = lc_var(a.order[p]);
+        a.pvs[at] = v;
+        a.c.pvrank[v] = at;
+        if (a.f_npvs) {  // one shared word per formula: counted no further than it is asked for
+            u32* n = &a.f_npvs[fid_of(a.c, v)];
+            if (vload(n) < a.lcve_min) atom_add(n, 1u);
+        }
+    }
+};
 
 }  // namespace sigma

@@ -143,14 +143,6 @@ HD void k_occurs_clause(const Ctx& c, u32 i) {
     }
 }
 
-// occurs straight from the occurrence-list sizes (valid when no clause changed since
-// the OT build): ps = |ot[2v]|, ns = |ot[2v+1]|.
-HD void k_occurs_from_ot(const Ctx& c, u32 v) {
-    if (v == 0) { c.ps[0] = c.ns[0] = 0; return; }
-    c.ps[v] = c.ot_size[V2L(v)];
-    c.ns[v] = c.ot_size[NEG(V2L(v))];
-}
-
 // ---------------------------------------------------------------- counts
 // countAll (src/cpu/solve.h:724-734): live clauses and their literals.
 struct CountArgs {

@@ -12,6 +12,15 @@
 
 namespace sigma {
 
+// The plain scan of an array (scan1_k's value and put).
+template <class Tin, class T>
+struct ScanArray {
+    const Tin* in;
+    T* out;
+    HD T value(size_t i) const { return (T)in[i]; }
+    HD void put(size_t i, T, T prefix) const { out[i] = prefix; }
+};
+
 #if SIGMA_CUDA
 
 constexpr int kScanThreads = 256;
@@ -143,9 +152,11 @@ constexpr int kScan1Items = 16;
 constexpr int kScan1Tile = kScanThreads * kScan1Items;
 __device__ __forceinline__ int scan1_pad(int i) { return i + (i >> 5); }
 
-template <class Tin, class T>
-__global__ void __launch_bounds__(kScanThreads) scan1_k(const Tin* in, T* out, size_t n, T* total, Scan1State st,
-                                                       u32 base, u32 epoch) {
+//
+// The scanned values come from f.value(i) and go to f.put(i, value, prefix), so a pass
+// that selects, ranks and writes items is one launch.
+template <class T, class F>
+__global__ void __launch_bounds__(kScanThreads) scan1_k(F f, size_t n, T* total, Scan1State st, u32 base, u32 epoch) {
     __shared__ T items[kScan1Tile + kScan1Tile / 32];
     __shared__ T ws[kScanThreads / 32];
     __shared__ u32 tile_s;
@@ -156,11 +167,13 @@ __global__ void __launch_bounds__(kScanThreads) scan1_k(const Tin* in, T* out, s
     const size_t nb = (n + kScan1Tile - 1) / kScan1Tile;
     const size_t t0 = (size_t)tile * kScan1Tile;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T own[kScan1Items];
 #pragma unroll
     for (int k = 0; k < kScan1Items; k++) {
         const int j = k * kScanThreads + threadIdx.x;
         const size_t i = t0 + (size_t)j;
-        items[scan1_pad(j)] = i < n ? (T)in[i] : T(0);
+        own[k] = i < n ? f.value(i) : T(0);
+        items[scan1_pad(j)] = own[k];
     }
     __syncthreads();
     // this thread's run: items [threadIdx.x * kScan1Items, +kScan1Items)
@@ -240,7 +253,7 @@ __global__ void __launch_bounds__(kScanThreads) scan1_k(const Tin* in, T* out, s
     for (int k = 0; k < kScan1Items; k++) {
         const int j = k * kScanThreads + threadIdx.x;
         const size_t i = t0 + (size_t)j;
-        if (i < n) out[i] = items[scan1_pad(j)];
+        if (i < n) f.put(i, own[k], items[scan1_pad(j)]);
     }
 }
 

@@ -39,7 +39,6 @@ struct FUpload { UploadArgs a; HD void operator()(u32 i) const { k_upload_clause
 struct FHist { Ctx c; HD void operator()(u32 i) const { k_hist_clause(c, i); } };
 struct FScatter { Ctx c; HD void operator()(u32 i) const { k_scatter_clause(c, i); } };
 struct FOccursCl { Ctx c; HD void operator()(u32 i) const { k_occurs_clause(c, i); } };
-struct FOccursOt { Ctx c; HD void operator()(u32 i) const { k_occurs_from_ot(c, i); } };
 struct FCount { CountArgs a; HD void operator()(u32 i) const { k_count_clause(a, i); } };
 struct FGcFlags { Ctx c; u32* keep; u64* sizes; HD void operator()(u32 i) const { k_gc_flags(c, keep, sizes, i); } };
 struct FGcMove { GcArgs a; HD void operator()(u32 i) const { k_gc_move(a, i); } };
@@ -48,21 +47,16 @@ struct FPropClause { PropArgs a; HD void operator()(u32 i) const { k_prop_clause
 struct FPropSweep { PropArgs a; HD void operator()(u32 i) const { k_prop_sweep(a, i); } };
 struct FPropSweepLists { PropArgs a; HD void operator()(u32 i) const { k_prop_sweep_lists(a, i); } };
 struct FReduce { Ctx c; HD void operator()(u32 i) const { k_reduce_list(c, i); } };
-struct FScores { LcveArgs a; u32* max_score; HD void operator()(u32 i) const { k_scores(a, max_score, i); } };
 struct FRank { LcveArgs a; HD void operator()(u32 i) const { k_rank(a, i); } };
-struct FMisRec { LcveArgs a; Q4* rec; HD void operator()(u32 i) const { k_mis_rec(a, rec, i); } };
 #if !SIGMA_CUDA
+struct FMisRec { LcveArgs a; Q4* rec; HD void operator()(u32 i) const { k_mis_rec(a, rec, i); } };
+struct FMisInit { LcveArgs a; MisFront b; HD void operator()(u32 i) const { k_mis_init(a, b, i); } };
 struct FMisPush { LcveArgs a; const u32* in; HD void operator()(u32 i) const { k_mis_push(a, in, i); } };
 struct FMisPull {
     LcveArgs a; const u32* in; MisFront und, ins; bool r0;
     HD void operator()(u32 i) const { k_mis_pull(a, in, und, ins, r0, i); }
 };
 #endif
-struct FMisInit { LcveArgs a; MisFront b; HD void operator()(u32 i) const { k_mis_init(a, b, i); } };
-struct FMisBound { LcveArgs a; HD void operator()(u32 i) const { k_mis_bound(a, i); } };
-struct FElectFlag { LcveArgs a; u32* flags; HD void operator()(u32 i) const { k_elect_flag(a, flags, i); } };
-struct FElectWrite { LcveArgs a; const u32* flags; const u32* scan; HD void operator()(u32 i) const { k_elect_write(a, flags, scan, i); } };
-struct FFill32 { u32* p; u32 v; HD void operator()(u32 i) const { p[i] = v; } };
 // Proof line of clause from + i (a resolvent just written).
 struct FProofClause {
     Ctx c; u32 from;
@@ -153,7 +147,6 @@ struct FPvKey {
         val[k] = k;
     }
 };
-struct FBoundInit { LcveArgs a; HD void operator()(u32 f) const { k_bound_init(a, f); } };
 struct FVarFid { u32* var_fid; const u32* f_var; u32 nf; HD void operator()(u32 v) const { k_var_fid(var_fid, f_var, nf, v); } };
 struct FCountFormula { FormulaCountArgs a; HD void operator()(u32 i) const { k_count_formula(a, i); } };
 // Batch partition of the elected list: group of each elected variable's formula
@@ -339,14 +332,13 @@ struct pf_sigma_ctx {
     DBuf<u64> counters64; // [0] nresolved, [2..3] counts
     DBuf<u64> ws_slots;   // [0, 32): elected lists' working set, [32, 64): graph working set (summed slots)
     // stage scratch
-    DBuf<u32> score, order, order_k2, order_v2, rank, bound, pvs, flags, flags_scan;
+    DBuf<u32> score, cand, order, order_k2, order_v2, rank, bound, pvs, flags, flags_scan;
     DBuf<u32> mis_big_a, mis_big_b;
     DBuf<u32> mis_word, mis_resume, mis_cmin;
 #if !SIGMA_CUDA
     DBuf<u32> mis_in[4];  // new-in lists of the serial election rounds (small x2, large x2)
 #endif
     DBuf<Q4> mis_rec;  // the election's 16-byte clause records
-    DBuf<u32> mis_gbits;  // the election's graph membership bitmap
     DBuf<u32> pv_perm, pv_key;
     DBuf<u32> work, cl_stamp;
     DBuf<u64> radix_work;
@@ -547,8 +539,8 @@ struct pf_sigma_ctx {
     // round: 200 variables 139 us at the full grid, 88 at 16 a variable, 121 at 4; 10k
     // variables 180, 141 and 195; from 100k variables on the grid is full at 4 or more
     // (100k: 469, 471, 469).
-    int mis_rounds_grid() {
-        return (int)std::min<u64>((u64)coop_grid(mis_rounds_k, mis_grid), ((u64)nvars * 16 + 255) / 256);
+    int mis_rounds_grid(u32 vars) {
+        return (int)std::max<u64>(std::min<u64>((u64)coop_grid(mis_rounds_k, mis_grid), ((u64)vars * 16 + 255) / 256), 1);
     }
 #endif
     void write_u64(u64* d, u64 v) { rt.h2d(d, &v, 8); }
@@ -571,6 +563,11 @@ struct pf_sigma_ctx {
     // the scan, its total written to the device word `total` (no synchronisation)
     template <class Tin, class T>
     void scan1_launch(const Tin* in, T* out, size_t n, T* total) {
+        scan_each(ScanArray<Tin, T>{in, out}, n, total);
+    }
+    // f.put(i, f.value(i), sum of the values before i) for i in [0, n)
+    template <class T, class F>
+    void scan_each(const F& f, size_t n, T* total) {
         const size_t tiles = scan1_tiles(n);
         if (!scan1_ctl.p || scan1_base > 0x7FFFFFFFu || scan1_epoch >= 0x3FFFFFFFu) {
             scan1_ctl.reserve(rt, 4);
@@ -591,8 +588,8 @@ struct pf_sigma_ctx {
         } else {
             Scan1State st{scan1_agg.p, scan1_incl.p, scan1_flag.p, scan1_ctl.p, counters.p + 1};
             rt.launches++;
-            scan1_k<Tin, T><<<(unsigned)tiles, kScanThreads, 0, rt.stream>>>(in, out, n, total, st, scan1_base,
-                                                                             ++scan1_epoch);
+            scan1_k<T, F><<<(unsigned)tiles, kScanThreads, 0, rt.stream>>>(f, n, total, st, scan1_base,
+                                                                           ++scan1_epoch);
             ck(cudaGetLastError(), "launch");
             scan1_base += (u32)tiles;
         }
@@ -601,6 +598,16 @@ struct pf_sigma_ctx {
     template <class Tin>
     u64 scan64(const Tin* in, u64* out, size_t n) { return scan1<Tin, u64>(in, out, n); }
 #else
+    template <class T, class F>
+    void scan_each(const F& f, size_t n, T* total) {
+        T t = 0;
+        for (size_t i = 0; i < n; i++) {
+            const T v = f.value(i);
+            f.put(i, v, t);
+            t += v;
+        }
+        *total = t;
+    }
     u32 scan32(const u32* in, u32* out, size_t n) {
         scan_tmp32.reserve(rt, scan_tmp_elems(n) + 2);
         u32* total = scan_tmp32.p + scan_tmp32.n - 1;
@@ -967,44 +974,53 @@ struct pf_sigma_ctx {
     // LCVE (lcve.cpp:46-81).
     bool lcve() {
         Ctx c = view();
-        rt.zero(ps.p, (size_t)(nvars + 1) * 4);
-        rt.zero(ns.p, (size_t)(nvars + 1) * 4);
-        if (ot_dirty) rt.each(FOccursCl{c}, ncls);
-        else rt.each(FOccursOt{c}, nvars + 1);
-        LcveArgs a;
+        if (ot_dirty) {
+            rt.zero(ps.p, (size_t)(nvars + 1) * 4);
+            rt.zero(ns.p, (size_t)(nvars + 1) * 4);
+            rt.each(FOccursCl{c}, ncls);
+        }
+        LcveArgs a{};
         a.c = c;
         a.pt = (u32)opt.mu_pos << mu_inc;
         a.nt = (u32)opt.mu_neg << mu_inc;
+        a.dirty = ot_dirty;
+        a.all = opt.dump_level >= 2;
         a.score = score.p;
+        a.cand = cand.p;
         a.order = order.p;
-        a.rank = rank.p;
+        a.key = order_k2.p;
+        a.max_score = counters.p + 27;
         a.word = mis_word.p;
         a.resume = mis_resume.p;
         mis_rec.reserve(rt, (size_t)ncls + 1);
         a.crec = mis_rec.p;
         mis_cmin.reserve(rt, (size_t)ncls + 1);
         a.cmin = mis_cmin.p;
-        mis_gbits.reserve(rt, (size_t)nvars / 32 + 1);
-        rt.zero(mis_gbits.p, ((size_t)nvars / 32 + 1) * 4);
-        a.gbits = mis_gbits.p;
         a.ws_bytes = ws_slots.p + kSpreadSlots;
         a.bound = bound.p;
         a.pvs = pvs.p;
         a.f_active = nf ? f_active.p : nullptr;
         a.f_npvs = nf ? f_npvs.p : nullptr;
-        const u32 nform = nf ? nf : 1u;
-        rt.zero(score.p, (size_t)(nvars + 1) * 4);
+        a.lcve_min = (u32)std::max(opt.lcve_min, 1);
+        a.nform = nf ? nf : 1u;
+        if (a.all) rt.zero(score.p, 4);
         rt.zero(counters.p + 27, 4);
-        rt.each(FScores{a, counters.p + 27}, nvars + 1);
+        scan_each(LcveCand{a}, nvars, (u32*)hslot(0));
+        word_to((u32*)hslot(0), 0);
+        word_to(counters.p + 27, 1);
+        read_slots_checked();
+        a.ncand = (u32)hr[0];
+        const u32 max_score = (u32)hr[1];
         // LCV order: stable by score over ascending variables (rSort, sort.h:123-133);
         // radix passes only over the bytes the largest score uses
-        const u32 max_score = read_u32(counters.p + 27);
         int bits = 8;
         while (bits < 32 && (max_score >> bits)) bits += 8;
-        rt.d2d(order_k2.p, score.p + 1, (size_t)nvars * 4);  // keys = score[1..]
-        sort_pairs(order_k2.p, order.p, order_v2.p, rank.p, nvars, bits);
-        rt.zero(bound.p, (size_t)nform * 8, 0xFF);
-        rt.each(FRank{a}, nvars);
+        radix_work.reserve(rt, radix_work_elems(a.ncand));
+        if (radix_sort_any(a.key, a.order, order_v2.p, rank.p, a.ncand, bits, radix_work.p, counters.p + 1, rt.stream,
+                           rt.launches))
+            a.order = rank.p;
+        rt.zero(bound.p, (size_t)a.nform * 8, 0xFF);
+        rt.each(FRank{a}, a.ncand);
         // Independent set by rounds. Undecided lists: flags|mis_big_a and
         // flags_scan|mis_big_b.
         mis_big_a.reserve(rt, nvars + 1);
@@ -1016,11 +1032,11 @@ struct pf_sigma_ctx {
         rt.zero(ctr, 15 * 4);
 #if SIGMA_CUDA
         rt.launches++;
-        mis_init_k<<<rt.grid(nvars + 1), 256, 0, rt.stream>>>(
-            a, MisFront{flags.p, ctr, mis_big_a.p, ctr + 1}, nvars + 1);
+        const u32 nitems = std::max(a.ncand, a.nform);
+        mis_init_k<<<rt.grid(nitems), 256, 0, rt.stream>>>(a, MisFront{flags.p, ctr, mis_big_a.p, ctr + 1}, nitems);
         ck(cudaGetLastError(), "launch");
 #else
-        rt.each(FMisInit{a, MisFront{flags.p, ctr, mis_big_a.p, ctr + 1}}, nvars + 1);
+        rt.each(FMisInit{a, MisFront{flags.p, ctr, mis_big_a.p, ctr + 1}}, std::max(a.ncand, a.nform));
 #endif
 #if SIGMA_CUDA
         if (ncls) {
@@ -1051,7 +1067,7 @@ struct pf_sigma_ctx {
         }
         void* args[] = {&a, &w};
         kclock[K_MIS].start(rt);
-        ck(cudaLaunchCooperativeKernel((const void*)mis_rounds_k, dim3(mis_rounds_grid()), dim3(256), args, 0,
+        ck(cudaLaunchCooperativeKernel((const void*)mis_rounds_k, dim3(mis_rounds_grid(a.ncand)), dim3(256), args, 0,
                                        rt.stream),
            "cooperative launch");
         kclock[K_MIS].stop(rt);
@@ -1074,14 +1090,12 @@ struct pf_sigma_ctx {
         }
         kclock[K_MIS].stop(rt);
 #endif
-        rt.each(FBoundInit{a}, nform);
-        rt.each(FMisBound{a}, nvars + 1);
-        rt.each(FFill32{pvrank.p, NONE}, nvars + 1);
-        rt.each(FElectFlag{a, flags.p}, nvars);
+        rt.zero(pvrank.p, ((size_t)nvars + 1) * 4, 0xFF);  // NONE
         if (nf) rt.zero(f_npvs.p, (size_t)nf * 4);
         // one read: the elected count, the rounds run and the error word (a round
-        // that ran out of time is caught here; the kernels since only read words)
-        scan_to(flags.p, flags_scan.p, nvars, 0);
+        // that ran out of time is caught here; the scan since only reads decided words)
+        scan_each(LcveElect{a}, a.ncand, (u32*)hslot(0));
+        word_to((u32*)hslot(0), 0);
 #if SIGMA_CUDA
         word_to(ctr + 14, 1);
 #endif
@@ -1092,7 +1106,6 @@ struct pf_sigma_ctx {
         if (trace_on) print_mis_trace(rounds);
 #endif
         mis_rounds += rounds;
-        rt.each(FElectWrite{a, flags.p, flags_scan.p}, nvars);
         n_go = npvs;
         perm_off = 0;
         perm_n = npvs;
@@ -1101,7 +1114,9 @@ struct pf_sigma_ctx {
         // stage dumps record an election that goes on (as the reference harness does)
         if (go && opt.dump_level >= 2) {
             rec(3, phase, 2, fetch(score.p, nvars + 1));
-            rec(4, phase, 2, fetch(order.p, nvars));
+            std::vector<u32> ord = fetch(a.order, nvars);
+            for (u32& x : ord) x = lc_var(x);
+            rec(4, phase, 2, ord);
         }
         if (go && opt.dump_level >= 1) rec(5, phase, 2, fetch(pvs.p, npvs));
         return go;
@@ -2239,7 +2254,8 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
         c.pvrank.reserve(rt, num_vars + 1);
         c.trail.reserve(rt, num_vars + 1);
         c.resolved.reserve(rt, (size_t)L + 2 * (size_t)num_vars + 4096);
-        c.score.reserve(rt, num_vars + 1);
+        if (c.opt.dump_level >= 2) c.score.reserve(rt, num_vars + 1);
+        c.cand.reserve(rt, num_vars + 1);
         c.order.reserve(rt, num_vars + 1);
         c.order_k2.reserve(rt, num_vars + 1);
         c.order_v2.reserve(rt, num_vars + 1);
