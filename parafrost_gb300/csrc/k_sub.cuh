@@ -152,46 +152,6 @@ HD void sub_strengthen(const SubArgs& a, u32 k, u32 p, u32 r, u32 me, SubLocal& 
     }
 }
 
-// subsume(list, end, cand) (subsume.h:105-121).
-HD bool sub_subsume(const Ctx& c, const u32* list, u32 end, u32 cr) {
-    const Hdr cand = c.hdr[cr];
-    const u32* cl = c.lits + cand.start;
-    for (u32 j = 0; j < end; j++) {
-        const u32 sr = list[j];
-        const Hdr s = c.hdr[sr];
-        if (h_deleted(s.flags)) continue;
-        if (h_molten(cand.flags) && s.size > cand.size) continue;
-        if (s.size > 1 && sig_sub(s.sig, cand.sig) && clause_sub(c.lits + s.start, s.size, cl, cand.size)) {
-            if (h_learnt(s.flags) && h_original(cand.flags)) {
-                c.hdr[sr].flags = (s.flags & ~3u) | ST_ORIGINAL;
-                touch(c, sr);
-            }
-            proof_delete(c, cr);
-            mark_deleted(c, cr);
-            return true;
-        }
-    }
-    return false;
-}
-
-// selfsubsume(x, fx, list, cand) (subsume.h:123-142).
-HD bool sub_selfsubsume(const SubArgs& a, u32 k, u32 p, u32 x, u32 fx, const u32* list, u32 ls, u32 cr, SubLocal& L) {
-    const Ctx& c = a.c;
-    const Hdr cand = c.hdr[cr];
-    const u32* cl = c.lits + cand.start;
-    for (u32 j = 0; j < ls; j++) {
-        const Hdr s = c.hdr[list[j]];
-        if (s.size > cand.size) break;
-        if (h_deleted(s.flags)) continue;
-        if (s.size > 1 && sig_selfsub(s.sig, cand.sig) && clause_selfsub(x, fx, c.lits + s.start, s.size, cl, cand.size)) {
-            sub_strengthen(a, k, p, cr, x, L);
-            set_molten(c, cr, true);
-            return true;
-        }
-    }
-    return false;
-}
-
 // updateOL (subsume.h:27-37).
 HD void sub_update_list(const Ctx& c, u32 l) {
     const u32 o = c.ot_off[l], s = c.ot_size[l];
@@ -203,43 +163,6 @@ HD void sub_update_list(const Ctx& c, u32 l) {
         else if (!h_deleted(f)) c.ot_refs[o + j++] = r;
     }
     c.ot_size[l] = j;
-}
-
-// self_sub_x (subsume.h:144-179), one elected variable per item.
-HD void k_sub_pv(const SubArgs& a, u32 k) {
-    if (a.run && !a.run[k]) return;
-    const Ctx& c = a.c;
-    const u32 v = a.pvs[k];
-    const u32 p = V2L(v), n = NEG(p);
-    if (c.ot_size[p] > a.sub_max || c.ot_size[n] > a.sub_max) return;
-    SubLocal L;
-    L.n = 0;
-    if (a.pre_off) {
-        for (u32 i = a.pre_off[k]; i < a.pre_off[k + 1]; i++) sub_local_oblivion(c, p, a.pre_lits[i]);
-    }
-    const u32* poss = c.ot_refs + c.ot_off[p];
-    const u32* negs = c.ot_refs + c.ot_off[n];
-    u32 ps = c.ot_size[p];
-    for (u32 i = 0; i < ps; i++) {
-        const u32 r = poss[i];
-        const Hdr h = c.hdr[r];
-        if (h.size > HSE_MAX_CL_SIZE) break;
-        if (h_deleted(h.flags)) continue;
-        sub_selfsubsume(a, k, p, p, n, negs, c.ot_size[n], r, L);
-        sub_subsume(c, poss, i, r);
-    }
-    sub_update_list(c, p);
-    ps = c.ot_size[p];
-    const u32 ns = c.ot_size[n];
-    for (u32 i = 0; i < ns; i++) {
-        const u32 r = negs[i];
-        const Hdr h = c.hdr[r];
-        if (h.size > HSE_MAX_CL_SIZE) break;
-        if (h_deleted(h.flags)) continue;
-        sub_selfsubsume(a, k, p, n, p, poss, c.ot_size[p], r, L);
-        sub_subsume(c, negs, i, r);
-    }
-    sub_update_list(c, n);
 }
 
 // Whether SUB on this variable can produce a unit: some binary (x u) in the

@@ -8,6 +8,15 @@
 // search over the earlier candidates (subsume.h:105-121: first clause that
 // subsumes it). Each takes the first hit in list order, so the outcome is the
 // sequential one. Writes to the clauses happen on lane 0 between warp barriers.
+//
+// For most variables nothing is subsumed or strengthened, and the loop is a chain of
+// two searches per candidate, each waiting for headers in memory. So the warp first
+// looks at all pairs of the two lists at once, with the headers staged in shared memory
+// (sub_nothing): when no pair as it stands would subsume or strengthen, no step of the
+// loop could change anything and only the deleted clauses leave the lists.
+// SUB of a round, before and now: 6.8M-clause AIG 2.49 and 1.38 ms, 80M community clauses
+// 8.8 and 6.8 (5M variables of 14 clauses), 384 mixed formulas 3.8 and 2.7, 10k 3-SAT 108
+// and 75 us.
 #pragma once
 
 #include "k_sub.cuh"
@@ -67,12 +76,74 @@ HD void sub_warp_side(const SubArgs& a, u32 k, u32 p, u32 lx, u32 lo, SubLocal& 
     wone([&] { sub_update_list(c, lx); });
 }
 
-HD void sub_warp_pv(const SubArgs& a, u32 k) {
+// Staged headers of a variable's two lists, entry after entry.
+constexpr u32 SUB_STAGE = 64;
+constexpr u32 SUB_SLOT = 4 * SUB_STAGE;  // words per warp
+
+// True when SUB changes no clause of the np + nn <= SUB_STAGE entries (its updateOL is
+// then done here); false leaves everything to the candidate loop. The pairs tested hold
+// every pair that the loop can act on as long as it has not acted: an earlier entry of
+// the same list that subsumes, an entry of the other list, no longer, that strengthens.
+HD bool sub_nothing(const Ctx& c, u32 p, u32 np, u32 nn, u32* slot) {
+    u32 *id = slot, *size = id + SUB_STAGE, *sig = size + SUB_STAGE, *start = sig + SUB_STAGE;
+    const u32 tot = np + nn;
+    u32* lp = c.ot_refs + c.ot_off[p];
+    u32* ln = c.ot_refs + c.ot_off[p + 1];
+    const u32 odd = wsum(tot, [&](u32 i) {  // deleted entries in the low half, molten ones in the high
+        const u32 r = i < np ? lp[i] : ln[i - np];
+        const Hdr h = c.hdr[r];
+        const bool dead = h_deleted(h.flags);
+        id[i] = r;
+        size[i] = dead ? 0u : h.size;  // no live clause is empty
+        sig[i] = h.sig;
+        start[i] = h.start;
+        return (dead ? 1u : 0u) + (h_molten(h.flags) ? 0x10000u : 0u);
+    });
+    wsync();
+    if (odd >> 16) return false;
+    const u32 inv = ((1u << 20) + tot - 1) / (tot ? tot : 1u);  // t / tot for t < 64 * 64
+    const u32 hit = wfirst(tot * tot, [&](u32 t) {
+        const u32 i = (t * inv) >> 20, j = t - i * tot;
+        const u32 si = size[i], sj = size[j];
+        if (sj < 2 || sj > si) return false;
+        const bool same = (i < np) == (j < np);
+        if (same) {
+            if (j >= i || !sig_sub(sig[j], sig[i])) return false;
+            return clause_sub(c.lits + start[j], sj, c.lits + start[i], si);
+        }
+        if (!sig_selfsub(sig[j], sig[i])) return false;
+        const u32 x = i < np ? p : NEG(p);
+        return clause_selfsub(x, FLIP(x), c.lits + start[j], sj, c.lits + start[i], si);
+    });
+    if (hit != NONE_IDX) return false;
+    if (!odd) return true;
+    // updateOL of both lists: the live entries move up in order
+    for (u32 side = 0; side < 2; side++) {
+        const u32 b = side ? np : 0u, n = side ? nn : np;
+        u32* l = side ? ln : lp;
+        u32 out = 0;
+        for (u32 base = 0; base < n; base += 32) {
+            const u32 m = wballot([&](u32 q) { return base + q < n && size[b + base + q] != 0; });
+            wfor(32, [&](u32 q) {
+                if ((m >> q) & 1u) l[out + (u32)popc32(m & ((1u << q) - 1u))] = id[b + base + q];
+            });
+            out += (u32)popc32(m);
+        }
+        wone([&] { c.ot_size[p + side] = out; });
+    }
+    return true;
+}
+
+HD void sub_warp_pv(const SubArgs& a, u32 k, u32* slot) {
     if (a.run && !a.run[k]) return;
     const Ctx& c = a.c;
     const u32 v = a.pvs[k];
     const u32 p = V2L(v), n = NEG(p);
-    if (c.ot_size[p] > a.sub_max || c.ot_size[n] > a.sub_max) return;
+    const u32 np = c.ot_size[p], nn = c.ot_size[n];
+    if (np > a.sub_max || nn > a.sub_max) return;
+    const bool pre = a.pre_off && a.pre_off[k] < a.pre_off[k + 1];
+    wsync();
+    if (!pre && np + nn <= SUB_STAGE && sub_nothing(c, p, np, nn, slot)) return;
     SubLocal L;  // lane 0's (only lane 0 strengthens)
     L.n = 0;
     if (a.pre_off) {
@@ -86,7 +157,9 @@ HD void sub_warp_pv(const SubArgs& a, u32 k) {
 
 #if SIGMA_CUDA
 // Warps take elected variables in work order (perm), a few at a time.
-__global__ void __launch_bounds__(256, 8) sub_warp_k(SubArgs a, const u32* perm, u32 n, u32* next) {
+__global__ void __launch_bounds__(256, 6) sub_warp_k(SubArgs a, const u32* perm, u32 n, u32* next) {
+    __shared__ u32 slots[8][SUB_SLOT];
+    u32* slot = slots[threadIdx.x >> 5];
     const u32 lane = threadIdx.x & 31u;
     u32 chunk = warp_chunk(n);
     while (true) {
@@ -95,7 +168,7 @@ __global__ void __launch_bounds__(256, 8) sub_warp_k(SubArgs a, const u32* perm,
         j0 = __shfl_sync(0xffffffffu, j0, 0);
         if (j0 >= n) break;
         const u32 j1 = j0 + chunk < n ? j0 + chunk : n;
-        for (u32 j = j0; j < j1; j++) sub_warp_pv(a, perm[j]);
+        for (u32 j = j0; j < j1; j++) sub_warp_pv(a, perm[j], slot);
         chunk = warp_chunk(n - j1);
     }
 }

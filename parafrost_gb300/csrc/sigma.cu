@@ -67,7 +67,6 @@ struct FProofClause {
 };
 struct FSortList { SortArgs a; HD void operator()(u32 i) const { k_sort_list(a, i); } };
 struct FSubPossible { SubArgs a; u32* flag; u32* prod; HD void operator()(u32 i) const { k_sub_unit_possible(a, flag, prod, i); } };
-struct FSubPv { SubArgs a; HD void operator()(u32 i) const { k_sub_pv(a, i); } };
 struct FSubNeed {
     Ctx c; const u32* pvs; const uint8_t* only; u32* ent; u64* words;
     HD void operator()(u32 i) const { k_sub_need(c, pvs, only, ent, words, i); }
@@ -95,7 +94,13 @@ struct FSubSave { SubCkptArgs a; HD void operator()(u32 i) const { k_sub_save(a,
 struct FSubRestore { SubCkptArgs a; HD void operator()(u32 i) const { k_sub_restore(a, i); } };
 struct FSubReach { SubReachArgs a; const u32* off; u32 nq; HD void operator()(u32 i) const { k_sub_reach(a, off, nq, i); } };
 struct FSubReachSize { Ctx c; const U2* units; u32* size; HD void operator()(u32 q) const { k_sub_reach_size(c, units, size, q); } };
-struct FSubWarp { SubArgs a; HD void operator()(u32 k) const { sub_warp_pv(a, k); } };
+struct FSubWarp {
+    SubArgs a;
+    HD void operator()(u32 k) const {
+        u32 slot[SUB_SLOT];
+        sub_warp_pv(a, k, slot);
+    }
+};
 struct FSubCommitSize { Ctx c; const u32* lits; u32* size; HD void operator()(u32 q) const { k_sub_commit_size(c, lits, size, q); } };
 struct FSubCommitItem {
     Ctx c; const u32* lits; const u32* off; u32 n;
