@@ -65,8 +65,8 @@ typedef struct {
                               * A small value exercises the give-up path without any wait. */
     int32_t proof;           /* "proof" = 0: 1 records the round's DRAT proof (pf_sigma_proof);
                               * single formulas only */
-    int32_t ot_buckets;      /* occurrence-table build: 0 by size (literal buckets once the
-                              * per-literal counters outgrow the L2 cache), 1 always literal
+    int32_t ot_buckets;      /* occurrence-table build: 0 by size (literal buckets once the table and its
+                              * counters outgrow 7/8 of the L2 cache), 1 always literal
                               * buckets, -1 always per-occurrence atomics */
     int32_t sweep_div;       /* propagation sweeps the whole store when the pending literals'
                               * lists exceed 1/sweep_div of it: 0 = 16, -1 never sweeps */

@@ -161,6 +161,65 @@ HD Hdr hdr_ro(const Hdr* p) {
     return *p;
 #endif
 }
+#if SIGMA_CUDA
+// The literals of 32 clauses (lane i's clause at `start`, `size` literals, 0: none)
+// walked by one warp, consecutive lanes on consecutive literals, 32 a step. Whose literal
+// a lane has is found by one reduction a step: the clauses that begin in the step's
+// window set their bits, and the owner is as many clauses on as bits are set up to the
+// lane (a search in the prefix took five shuffles a step). Lanes without a clause would
+// have no place of their own in the window, so the others are first moved together.
+// Instructions for 32 literals of the table build's fill, two walks: 204 before, @WALK@.
+struct WarpWalk {
+    u32 excl, incl, total;  // this lane's clause: first and past-the-last place in the walk
+
+    DEV void init(u32 start, u32 size) {
+        const u32 lane = threadIdx.x & 31u;
+        incl = size;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u32 t = __shfl_up_sync(kFull, incl, o);
+            if ((int)lane >= o) incl += t;
+        }
+        excl = incl - size;
+        total = __shfl_sync(kFull, incl, 31);
+        before = 0;
+        from = lane;
+        first = excl;
+        adj = start - excl;
+        const u32 have = __ballot_sync(kFull, size != 0);
+        if (have != kFull) {
+            u32 r = lane, pos = 0;  // the place of the lane-th set bit
+#pragma unroll
+            for (u32 w = 16; w; w >>= 1) {
+                const u32 c = (u32)__popc((have >> pos) & ((1u << w) - 1u));
+                if (c <= r) {
+                    r -= c;
+                    pos += w;
+                }
+            }
+            from = pos & 31u;
+            first = __shfl_sync(kFull, excl, (int)from);
+            adj = __shfl_sync(kFull, adj, (int)from);
+            if (lane >= (u32)__popc(have)) first = 0xFFFFFFFFu;
+        }
+    }
+    // Step `base` (0, 32, 64, ...): the lane whose clause holds place base + lane, and
+    // the literal's index in the store (both only where base + lane < total).
+    DEV void step(u32 base, u32& owner, u32& src) {
+        const u32 lane = threadIdx.x & 31u;
+        const u32 off = first - base;
+        const u32 m = __reduce_or_sync(kFull, off < 32u ? 1u << off : 0u);
+        const u32 k = before + (u32)__popc(m & ((2u << lane) - 1u)) - 1u;
+        before += (u32)__popc(m);
+        owner = __shfl_sync(kFull, from, (int)(k & 31u));
+        src = __shfl_sync(kFull, adj, (int)(k & 31u)) + base + lane;
+    }
+
+   private:
+    u32 before;             // clauses that begin before the step
+    u32 from, first, adj;   // the lane-th clause that has literals: its lane, place, start less place
+};
+#endif
 HD const u32* clause_lits(const Ctx& c, const Hdr& h) { return c.lits + h.start; }
 
 // Signature of a literal array.

@@ -8,14 +8,20 @@
 //     one to its bucket in a per-block shared histogram; one atomic per bucket per
 //     block at the end. An exclusive scan of the bucket counts gives every bucket
 //     its range of the table (all its literals' lists, side by side).
-//   pass 1 (ot_bucket_fill_k): per tile of clauses, every occurrence (literal,
-//     clause id, one 8-byte word) is staged in shared memory and counted per
-//     bucket; a block scan orders the tile by bucket, one reservation per non-empty
-//     bucket gives each run its place, and the runs are written out contiguously
-//     (consecutive threads on consecutive words).
+//   pass 1 (ot_bucket_fill_k): per tile of clauses, the occurrences are counted per
+//     bucket, one reservation per non-empty bucket gives each run its place, a block scan
+//     orders the tile by bucket, the occurrences are staged in shared memory in that order
+//     (slot in its bucket and clause in its tile: one word) and every run is written out by
+//     a warp, clause ids and slots side by side (6 bytes an occurrence).
 //   pass 2 (ot_bucket_lists_k): one block per bucket: per-slot counts in shared
-//     memory, a block scan gives the list sizes and starts of the bucket's slots,
-//     then every occurrence lands in its list inside the bucket's range.
+//     memory (from the 2-byte slots alone), a block scan gives the list sizes and starts of
+//     the bucket's slots, then every occurrence lands in its list inside the bucket's range.
+// What bounds it: pass 1 the issue slots of its two walks (74% busy on 28M occurrences,
+// 252 us; 295 us when whose literal a lane has was searched for in five shuffles a step),
+// pass 2 the scattered 4-byte stores. All tables of a round, before (6,144 occurrences a
+// tile staged as 8-byte pairs) and now: 80M community clauses 14.6 and 13.8 ms, 8M 1.41 and
+// 1.31. Tiles of 6,144, 8,192, 14,336 and 30,720 occurrences with 4, 3, 2 and 1 blocks an
+// SM: 14.9, 14.4, 13.8 and 14.1 ms.
 // Clause headers and literals are read by whole warps, consecutive lanes on
 // consecutive literals. The order inside one list is unspecified, as for the
 // atomic build: the elected lists are sorted into the reference's order later.
@@ -27,13 +33,15 @@ namespace sigma {
 
 #if SIGMA_CUDA
 
-constexpr u32 OTB_TILE = 4096;      // clauses per block tile in pass 0
-constexpr u32 OTB_FILL_CAP = 6144;   // occurrences of a pass-1 tile ordered in shared memory
-                                     // (48 KB: three 512-thread blocks per SM)
+constexpr u32 OTB_FILL_CAP = 14336;  // occurrences of a pass-1 tile ordered in shared memory
+                                     // (84 KB: two blocks per SM)
+constexpr u32 OTB_MAX_TILE = 1u << 16;  // clauses of a pass-1 tile
 constexpr u32 OTB_MAX_BUCKETS = 4096;
 constexpr u32 OTB_MAX_SHIFT = 15;   // 32,768 slots: 128 KiB of shared counters in pass 2
 constexpr u32 OTB_LIST_THREADS = 1024;  // one block a bucket, 32 warps to keep its loads in flight
 constexpr unsigned OTB_FULL = 0xffffffffu;
+// (clause in the tile, slot) in one word
+static_assert(OTB_MAX_SHIFT <= 15 && OTB_MAX_TILE <= 1u << 17, "a staged occurrence is one word");
 
 struct OtbArgs {
     Ctx c;
@@ -42,47 +50,51 @@ struct OtbArgs {
     u32* count;       // nb: occurrences per bucket (pass 0)
     u32* cursor;      // nb: next free position of every bucket (pass 1; starts at base)
     const u32* base;  // nb + 1: first position of every bucket, base[nb] = occurrences
-    u64* tpair;       // occurrences grouped by bucket: clause id << 32 | literal
+    u32* tcid;        // occurrences grouped by bucket: clause ids
+    unsigned short* tslot;  // and literals, less the bucket's first
     u32 fill_tile;    // clauses per pass-1 tile (a multiple of 32)
 };
 
-// The literals of the live clauses id0 .. id0+n-1 (n <= 32), walked by one warp with
-// consecutive lanes on consecutive literals (clauses are mostly adjacent in the
-// literal array, so the loads coalesce). f(valid, literal, clause id) is called by
-// every lane of the warp in every step, valid false past the end.
+// The literals of the live clauses c0 .. c1-1, walked by the warps of a block (warp w of nw
+// takes every nw-th group of 32 clauses), consecutive lanes on consecutive literals
+// (clauses are mostly adjacent in the literal array, so the loads coalesce).
+// f(literal, clause id) is called by the lanes that have one. Four steps' loads and the
+// next group's headers are in flight together: a walk waits for memory once a group, not
+// once a step. Returns the number of literals this warp walked.
 template <class F>
-DEV void warp_clause_literals(const Ctx& c, u32 id0, u32 n, F&& f) {
+DEV u32 warp_clause_literals(const Ctx& c, u32 c0, u32 c1, u32 w, u32 nw, F&& f) {
     const u32 lane = threadIdx.x & 31u;
-    u32 start = 0, sz = 0;
-    if (lane < n) {
-        const Hdr h = hdr_ro(&c.hdr[id0 + lane]);
-        if (!h_deleted(h.flags)) {
-            start = h.start;
-            sz = h.size;
+    auto header = [&](u32 g, u32& start, u32& size) {
+        start = size = 0;
+        if (g < c1 && lane < c1 - g) {
+            const Hdr h = hdr_ro(&c.hdr[g + lane]);
+            if (!h_deleted(h.flags)) {
+                start = h.start;
+                size = h.size;
+            }
+        }
+    };
+    u32 sum = 0, start, size;
+    header(c0 + w * 32u, start, size);
+    for (u32 g = c0 + w * 32u; g < c1; g += nw * 32u) {
+        WarpWalk ww;
+        ww.init(start, size);
+        header(g + nw * 32u, start, size);
+        sum += ww.total;
+        for (u32 base = 0; base < ww.total; base += 128) {
+            u32 k[4], l[4];
+#pragma unroll
+            for (u32 q = 0; q < 4; q++) {
+                u32 src;
+                if (base + 32u * q < ww.total) ww.step(base + 32u * q, k[q], src);
+                if (base + 32u * q + lane < ww.total) l[q] = __ldg(&c.lits[src]);
+            }
+#pragma unroll
+            for (u32 q = 0; q < 4; q++)
+                if (base + 32u * q + lane < ww.total) f(l[q], g + k[q]);
         }
     }
-    u32 incl = sz;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const u32 t = __shfl_up_sync(OTB_FULL, incl, o);
-        if ((int)lane >= o) incl += t;
-    }
-    const u32 excl = incl - sz;
-    const u32 total = __shfl_sync(OTB_FULL, incl, 31);
-    for (u32 base = 0; base < total; base += 32) {
-        const u32 j = base + lane;
-        // owner: the first lane k whose inclusive end is past j
-        u32 k = 0;
-#pragma unroll
-        for (u32 step = 16; step; step >>= 1) {
-            const u32 v = __shfl_sync(OTB_FULL, incl, k + step - 1);
-            if (v <= j) k += step;
-        }
-        const u32 st = __shfl_sync(OTB_FULL, start, k & 31u), ex = __shfl_sync(OTB_FULL, excl, k & 31u);
-        const bool valid = j < total;
-        const u32 lit = valid ? __ldg(&c.lits[st + (j - ex)]) : 0u;
-        f(valid, lit, id0 + k);
-    }
+    return sum;
 }
 
 // Pass 0: occurrences per bucket.
@@ -90,15 +102,9 @@ __global__ void __launch_bounds__(256) ot_bucket_count_k(OtbArgs a) {
     extern __shared__ u32 otb_hist[];
     for (u32 b = threadIdx.x; b < a.nb; b += blockDim.x) otb_hist[b] = 0;
     __syncthreads();
-    const u32 warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const u32 ngroups = (a.c.ncls + 31u) / 32u;
-    for (u32 g = blockIdx.x * nw + warp; g < ngroups; g += gridDim.x * nw) {
-        const u32 id0 = g * 32u;
-        const u32 n = a.c.ncls - id0 < 32u ? a.c.ncls - id0 : 32u;
-        warp_clause_literals(a.c, id0, n, [&](bool valid, u32 lit, u32) {
-            if (valid) atomicAdd(&otb_hist[lit >> a.shift], 1u);
-        });
-    }
+    const u32 nw = blockDim.x >> 5;
+    warp_clause_literals(a.c, 0, a.c.ncls, blockIdx.x * nw + (threadIdx.x >> 5), gridDim.x * nw,
+                         [&](u32 lit, u32) { atomicAdd(&otb_hist[lit >> a.shift], 1u); });
     __syncthreads();
     for (u32 b = threadIdx.x; b < a.nb; b += blockDim.x)
         if (otb_hist[b]) atomicAdd(&a.count[b], otb_hist[b]);
@@ -131,66 +137,62 @@ DEV u32 otb_block_scan(u32* cnt, u32 n, u32* warp_tot, u32* carry) {
     return *carry;
 }
 
-// Pass 1: occurrences grouped by bucket. A tile's occurrences are counted per
-// bucket (shared counters), one reservation per non-empty bucket gives each run its
-// place, a block scan of the counts orders the tile by bucket, and a second walk of
-// the tile's literals (just read, so mostly cache hits) places every occurrence in
-// shared memory at its bucket's position; the runs are then written out contiguously.
-// A tile with more occurrences than shared memory holds (very long clauses) writes
-// them to their runs directly instead. Tiles hold fill_tile clauses, sized from the
-// mean clause length so that a tile's occurrences nearly fill the stage.
-constexpr u32 OTB_FILL_THREADS = 512;
-__global__ void __launch_bounds__(OTB_FILL_THREADS) ot_bucket_fill_k(OtbArgs a) {
-    extern __shared__ u64 otb_fsm[];
-    u64* sorted = otb_fsm;                                      // OTB_FILL_CAP
-    u32* cnt = reinterpret_cast<u32*>(otb_fsm + OTB_FILL_CAP);  // nb: counts, then tile offsets
-    u32* run = cnt + a.nb;                                      // nb: global start of the tile's run
-    u32* cur = run + a.nb;                                      // nb: cursors
+// Pass 1: occurrences grouped by bucket. The tile's literals are walked twice (the second
+// time mostly cache hits): once to count them per bucket, once to place them. A tile with
+// more occurrences than shared memory holds (very long clauses) writes them to their runs
+// directly instead. Tiles hold fill_tile clauses, sized from the mean clause length so
+// that a tile's occurrences nearly fill the stage.
+constexpr u32 OTB_FILL_THREADS = 768;
+__global__ void __launch_bounds__(OTB_FILL_THREADS, 2) ot_bucket_fill_k(OtbArgs a) {
+    extern __shared__ u32 otb_fsm[];
+    u32* stage = otb_fsm;              // OTB_FILL_CAP: clause in the tile << OTB_MAX_SHIFT | slot
+    unsigned short* bucket = reinterpret_cast<unsigned short*>(stage + OTB_FILL_CAP);  // OTB_FILL_CAP
+    u32* cur = stage + OTB_FILL_CAP + OTB_FILL_CAP / 2;  // nb: counts, then places
+    u32* run = cur + a.nb;                               // nb: global start of the tile's run, less its place
     __shared__ u32 warp_tot[OTB_FILL_THREADS / 32];
     __shared__ u32 carry, ntile;
-    const u32 warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const u32 T = a.fill_tile;
+    const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const u32 T = a.fill_tile, smask = (1u << a.shift) - 1u;
     const u32 ntiles = (a.c.ncls + T - 1u) / T;
     for (u32 t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const u32 c0 = t * T, c1 = a.c.ncls - c0 < T ? a.c.ncls : c0 + T;
-        for (u32 b = threadIdx.x; b < a.nb; b += blockDim.x) cnt[b] = 0;
+        for (u32 b = threadIdx.x; b < a.nb; b += blockDim.x) cur[b] = 0;
         if (threadIdx.x == 0) ntile = 0;
         __syncthreads();
-        for (u32 g = c0 + warp * 32u; g < c1; g += nw * 32u)
-            warp_clause_literals(a.c, g, c1 - g < 32u ? c1 - g : 32u, [&](bool valid, u32 lit, u32) {
-                const unsigned m = __ballot_sync(OTB_FULL, valid);
-                if ((threadIdx.x & 31u) == 0 && m) atomicAdd(&ntile, (u32)__popc(m));
-                if (valid) atomicAdd(&cnt[lit >> a.shift], 1u);
-            });
+        const u32 nwarp = warp_clause_literals(a.c, c0, c1, warp, nw,
+                                               [&](u32 lit, u32) { atomicAdd(&cur[lit >> a.shift], 1u); });
+        if (lane == 0 && nwarp) atomicAdd(&ntile, nwarp);
         __syncthreads();
         const u32 n = ntile;
         for (u32 b = threadIdx.x; b < a.nb; b += blockDim.x) {
-            const u32 k = cnt[b];
+            const u32 k = cur[b];
             run[b] = k ? atomicAdd(&a.cursor[b], k) : 0u;
         }
         if (n <= OTB_FILL_CAP) {
-            otb_block_scan(cnt, a.nb, warp_tot, &carry);
-            for (u32 b = threadIdx.x; b < a.nb; b += blockDim.x) cur[b] = cnt[b];
+            otb_block_scan(cur, a.nb, warp_tot, &carry);
+            for (u32 b = threadIdx.x; b < a.nb; b += blockDim.x) run[b] -= cur[b];
             __syncthreads();
-            for (u32 g = c0 + warp * 32u; g < c1; g += nw * 32u)
-                warp_clause_literals(a.c, g, c1 - g < 32u ? c1 - g : 32u, [&](bool valid, u32 lit, u32 cid) {
-                    if (valid) sorted[atomicAdd(&cur[lit >> a.shift], 1u)] = ((u64)cid << 32) | lit;
-                });
+            warp_clause_literals(a.c, c0, c1, warp, nw, [&](u32 lit, u32 cid) {
+                const u32 b = lit >> a.shift, q = atomicAdd(&cur[b], 1u);
+                stage[q] = (cid - c0) << OTB_MAX_SHIFT | (lit & smask);
+                bucket[q] = (unsigned short)b;
+            });
             __syncthreads();
             for (u32 i = threadIdx.x; i < n; i += blockDim.x) {
-                const u64 x = sorted[i];
-                const u32 b = (u32)x >> a.shift;
-                a.tpair[run[b] + (i - cnt[b])] = x;
+                const u32 x = stage[i], q = run[bucket[i]] + i;
+                a.tcid[q] = c0 + (x >> OTB_MAX_SHIFT);
+                a.tslot[q] = (unsigned short)(x & ((1u << OTB_MAX_SHIFT) - 1u));
             }
         } else {
+            __syncthreads();
             for (u32 b = threadIdx.x; b < a.nb; b += blockDim.x) cur[b] = 0;
             __syncthreads();
-            for (u32 g = c0 + warp * 32u; g < c1; g += nw * 32u)
-                warp_clause_literals(a.c, g, c1 - g < 32u ? c1 - g : 32u, [&](bool valid, u32 lit, u32 cid) {
-                    if (!valid) return;
-                    const u32 b = lit >> a.shift;
-                    a.tpair[run[b] + atomicAdd(&cur[b], 1u)] = ((u64)cid << 32) | lit;
-                });
+            warp_clause_literals(a.c, c0, c1, warp, nw, [&](u32 lit, u32 cid) {
+                const u32 b = lit >> a.shift;
+                const u32 q = run[b] + atomicAdd(&cur[b], 1u);
+                a.tcid[q] = cid;
+                a.tslot[q] = (unsigned short)(lit & smask);
+            });
         }
         __syncthreads();
     }
@@ -210,18 +212,18 @@ __global__ void __launch_bounds__(OTB_LIST_THREADS) ot_bucket_lists_k(OtbArgs a)
     for (u32 i = tid; i < nl; i += blockDim.x) otb_cnt[i] = 0;
     if (tid == 0) carry = 0;
     __syncthreads();
-    // four occurrences per thread per step, their loads issued before the atomics; the
-    // staged pairs are read twice and then dead (evicted first), the lists' lines are
-    // filled by scattered stores and kept while they fill
+    // four consecutive occurrences per thread per step, in one load each; the staged
+    // words are read for the last time in the second walk (evicted first), the lists'
+    // lines are filled by scattered stores and kept while they fill
     const u64 pf = l2_policy_first(), pl = l2_policy_last();
     const u32 step = 4u * blockDim.x;
-    for (u32 k0 = p0 + tid; k0 < p1; k0 += step) {
-        u64 x[4];
-#pragma unroll
-        for (u32 j = 0; j < 4; j++) x[j] = k0 + j * blockDim.x < p1 ? ldcg_hint64(&a.tpair[k0 + j * blockDim.x], pf) : 0ull;
-#pragma unroll
-        for (u32 j = 0; j < 4; j++)
-            if (k0 + j * blockDim.x < p1) atomicAdd(&otb_cnt[(u32)x[j] - l0], 1u);
+    const u32 a0 = p0 & ~3u;  // the arrays are 16-byte aligned
+    for (u32 k0 = a0 + 4u * tid; k0 < p1; k0 += step) {
+        const ushort4 x = __ldcg(reinterpret_cast<const ushort4*>(a.tslot + k0));
+        if (k0 >= p0) atomicAdd(&otb_cnt[x.x], 1u);
+        if (k0 + 1 >= p0 && k0 + 1 < p1) atomicAdd(&otb_cnt[x.y], 1u);
+        if (k0 + 2 >= p0 && k0 + 2 < p1) atomicAdd(&otb_cnt[x.z], 1u);
+        if (k0 + 3 >= p0 && k0 + 3 < p1) atomicAdd(&otb_cnt[x.w], 1u);
     }
     __syncthreads();
     // block scan of the slot counts, blockDim.x slots per step: list sizes and starts
@@ -248,14 +250,14 @@ __global__ void __launch_bounds__(OTB_LIST_THREADS) ot_bucket_lists_k(OtbArgs a)
         if (tid == blockDim.x - 1) carry = excl + v;
         __syncthreads();
     }
-    for (u32 k0 = p0 + tid; k0 < p1; k0 += step) {
-        u64 x[4];
-#pragma unroll
-        for (u32 j = 0; j < 4; j++) x[j] = k0 + j * blockDim.x < p1 ? ldcg_hint64(&a.tpair[k0 + j * blockDim.x], pf) : 0ull;
-#pragma unroll
-        for (u32 j = 0; j < 4; j++)
-            if (k0 + j * blockDim.x < p1)
-                st_hint(&a.c.ot_refs[p0 + atomicAdd(&otb_cnt[(u32)x[j] - l0], 1u)], (u32)(x[j] >> 32), pl);
+    for (u32 k0 = a0 + 4u * tid; k0 < p1; k0 += step) {
+        const ushort4 x = __ldcg(reinterpret_cast<const ushort4*>(a.tslot + k0));
+        const Q4 id = ldro4_hint(reinterpret_cast<const Q4*>(a.tcid + k0), pf);
+        u32* refs = a.c.ot_refs + p0;
+        if (k0 >= p0) st_hint(&refs[atomicAdd(&otb_cnt[x.x], 1u)], id.x, pl);
+        if (k0 + 1 >= p0 && k0 + 1 < p1) st_hint(&refs[atomicAdd(&otb_cnt[x.y], 1u)], id.y, pl);
+        if (k0 + 2 >= p0 && k0 + 2 < p1) st_hint(&refs[atomicAdd(&otb_cnt[x.z], 1u)], id.z, pl);
+        if (k0 + 3 >= p0 && k0 + 3 < p1) st_hint(&refs[atomicAdd(&otb_cnt[x.w], 1u)], id.w, pl);
     }
 }
 

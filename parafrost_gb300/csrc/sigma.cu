@@ -744,14 +744,19 @@ struct pf_sigma_ctx {
     // ------------------------------------------------------------ stages
 #if SIGMA_CUDA
     // Occurrence table by literal buckets (k_otb.cuh): buckets of 2^shift literal
-    // slots, at most OTB_MAX_BUCKETS of them (so up to 134M literal slots). Used when
-    // the per-literal counters (4 bytes a slot) outgrow the L2 cache, where the
-    // atomic histogram and scatter turn into random device-memory traffic.
-    static constexpr u64 kOtbMinSlots = 1ull << 24;
+    // slots, at most OTB_MAX_BUCKETS of them (so up to 134M literal slots). Used when the
+    // table and its counters (4 bytes an occurrence and a slot) outgrow 7/8 of the L2
+    // cache, where the atomic histogram and scatter turn into random device-memory
+    // traffic. Tables of a round, atomics and buckets: 3-SAT with 12.6M occurrences 1.10
+    // and 1.05 ms, with 37.8M 5.6 and 2.9; community formulas with 21M 1.10 and 1.03, 28M
+    // 1.64 and 1.30, 56M 4.7 and 2.4; AIGs, whose clauses name neighbouring variables,
+    // with 16.4M 1.28 and 1.71, 33M 2.74 and 3.09, 66M 6.4 and 6.3.
+    static constexpr u64 kOtbMinBytes = 7ull << 24;
     DBuf<u32> otb_count, otb_base, otb_cursor;
-    DBuf<u64> otb_pair;
+    DBuf<u32> otb_cid;
+    DBuf<unsigned short> otb_slot;
     bool otb_plan(u32& shift, u32& nb) const {
-        if (opt.ot_buckets < 0 || (opt.ot_buckets == 0 && D < kOtbMinSlots)) return false;
+        if (opt.ot_buckets < 0 || (opt.ot_buckets == 0 && 4ull * (nlits_used + D) < kOtbMinBytes)) return false;
         u32 s = 8;
         while (s < OTB_MAX_SHIFT && ((u64)D >> s) > 1024) s++;
         shift = s;
@@ -762,20 +767,24 @@ struct pf_sigma_ctx {
         otb_count.reserve(rt, nb + 1);
         otb_base.reserve(rt, nb + 1);
         otb_cursor.reserve(rt, nb + 1);
-        otb_pair.reserve(rt, (size_t)nlits_used + 1);
+        otb_cid.reserve(rt, (size_t)nlits_used + 4);
+        otb_slot.reserve(rt, (size_t)nlits_used + 4);
         rt.zero(otb_count.p, (size_t)nb * 4);
         // pass-1 tiles: about 7/8 of the stage at the store's mean clause length
         const u64 mean_x8 = std::max<u64>(8ull * nlits_used / std::max<u32>(ncls, 1), 8);
-        const u32 fill_tile = (u32)std::min<u64>(std::max<u64>(7ull * OTB_FILL_CAP / mean_x8, 32), 4096) & ~31u;
-        OtbArgs a{view(), shift, nb, otb_count.p, otb_cursor.p, otb_base.p, otb_pair.p, fill_tile};
-        const u32 fill_smem = OTB_FILL_CAP * 8 + 3 * nb * 4;
+        // (fewer on a store too small to give every resident block four tiles)
+        const u64 by_stage = 7ull * OTB_FILL_CAP / mean_x8, by_grid = ncls / (8ull * (u32)rt.sms);
+        const u32 fill_tile =
+            (u32)std::min<u64>(std::max<u64>(std::min(by_stage, by_grid), 32), OTB_MAX_TILE) & ~31u;
+        OtbArgs a{view(), shift, nb, otb_count.p, otb_cursor.p, otb_base.p, otb_cid.p, otb_slot.p, fill_tile};
+        const u32 fill_smem = OTB_FILL_CAP * 6 + 2 * nb * 4;
         static bool attr_set = false;
         if (!attr_set) {
             ck(cudaFuncSetAttribute(ot_bucket_lists_k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)((1u << OTB_MAX_SHIFT) * 4)),
                "smem attr");
             ck(cudaFuncSetAttribute(ot_bucket_fill_k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(OTB_FILL_CAP * 8 + 3 * OTB_MAX_BUCKETS * 4)),
+                                    (int)(OTB_FILL_CAP * 6 + 2 * OTB_MAX_BUCKETS * 4)),
                "smem attr");
             attr_set = true;
         }
