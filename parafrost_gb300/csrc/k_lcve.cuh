@@ -16,6 +16,7 @@
 #pragma once
 
 #include "cnf.cuh"
+#include "prims.cuh"
 
 namespace sigma {
 
@@ -80,15 +81,18 @@ HD u32 lcve_ns(const LcveArgs& a, u32 v) { return a.dirty ? a.c.ns[v] : a.c.ot_s
 constexpr u32 MIS_WARP_MIN_OCC = 32;
 struct LcveCand {
     LcveArgs a;
-    HD u32 value(size_t i) const {
+    struct State { u32 max_score = 0; };
+    static constexpr int kItems = 8;
+    HD u32 value(size_t i, State& st) const {
         const u32 v = (u32)i + 1u;
         const u32 p = lcve_ps(a, v), n = lcve_ns(a, v);
         const bool valid = (p || n) && !a.c.vstate[v] && (!a.f_active || a.f_active[fid_of(a.c, v)]);
         a.word[v] = MIS_NO_RANK;
         if (a.all) a.score[v] = p * n;
-        warp_max_atomic(a.max_score, valid || a.all ? p * n : 0u);
+        if ((valid || a.all) && p * n > st.max_score) st.max_score = p * n;
         return valid || a.all;
     }
+    HD void done(const State& st) const { warp_max_atomic(a.max_score, st.max_score); }
     HD void put(size_t i, u32 take, u32 at) const {
         if (!take) return;
         const u32 v = (u32)i + 1u;
@@ -691,7 +695,10 @@ __global__ void __launch_bounds__(256, 6) mis_rounds_k(LcveArgs a0, MisRounds w)
 // order. One scan over the order.
 struct LcveElect {
     LcveArgs a;
-    HD u32 value(size_t p) const {
+    typedef ScanNone State;
+    static constexpr int kItems = 8;
+    HD void done(const State&) const {}
+    HD u32 value(size_t p, State&) const {
         const u32 v = lc_var(a.order[p]);
         const u32 w = a.word[v];
         return (u32)p < a.bound[2 * fid_of(a.c, v) + 1] && mis_rank(w) != MIS_NO_RANK && mis_dec(w) == MIS_IN;

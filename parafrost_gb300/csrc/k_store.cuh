@@ -4,6 +4,7 @@
 
 #include "cnf.cuh"
 #include "introsort.cuh"
+#include "prims.cuh"
 
 namespace sigma {
 
@@ -31,6 +32,37 @@ struct UploadArgs {
     const u32* f_nv;
 };
 
+// A short clause sorted in registers (an in-place sort waits for memory at every swap):
+// all literals loaded together, a transposition network, a store where the order changed.
+// Returns whether a literal is out of range or a variable repeated; sig is its signature.
+// (Device-side upload of 80M community clauses 3.4 ms in place, 2.2 with the short ones in
+// registers.)
+constexpr u32 UPLOAD_SHORT = 8;
+HD u32 upload_short(u32* l, u32 n, u32 D, u32& sig) {
+    u32 x[UPLOAD_SHORT], y[UPLOAD_SHORT];
+#pragma unroll
+    for (u32 k = 0; k < UPLOAD_SHORT; k++) x[k] = y[k] = k < n ? l[k] : 0xFFFFFFFFu;
+    // odd-even transposition: UPLOAD_SHORT rounds sort any order
+#pragma unroll
+    for (u32 r = 0; r < UPLOAD_SHORT; r++) {
+#pragma unroll
+        for (u32 k = r & 1u; k + 1 < UPLOAD_SHORT; k += 2) {
+            const u32 lo = y[k] < y[k + 1] ? y[k] : y[k + 1], hi = y[k] < y[k + 1] ? y[k + 1] : y[k];
+            y[k] = lo;
+            y[k + 1] = hi;
+        }
+    }
+    u32 bad = 0;
+#pragma unroll
+    for (u32 k = 0; k < UPLOAD_SHORT; k++) {
+        if (k >= n) continue;
+        bad |= y[k] < 2 || y[k] >= D || (k && ABS(y[k]) == ABS(y[k ? k - 1 : 0]));
+        sig |= MAPHASH(y[k]);
+        if (y[k] != x[k]) l[k] = y[k];
+    }
+    return bad;
+}
+
 HD void k_upload_clause(const UploadArgs& a, u32 i) {
     const u64 o0 = a.off[i], o1 = a.off[i + 1];
     // offsets that go down, or leave the uploaded literals, are rejected before
@@ -48,15 +80,18 @@ HD void k_upload_clause(const UploadArgs& a, u32 i) {
             l[k] += shift;
         }
     }
-    if (n <= 32) ref_insertion_sort(l, (int)n, LitLess());
-    else std_sort_replica(l, l + n, LitLess());
-    u32 sig = 0;
-    for (u32 k = 0; k < n; k++) {
-        const u32 lit = l[k];
-        if (lit < 2 || lit >= a.c.D) { set_err(a.c, ERR_INPUT); return; }
-        if (k && ABS(lit) == ABS(l[k - 1])) { set_err(a.c, ERR_INPUT); return; }
-        sig |= MAPHASH(lit);
+    u32 sig = 0, bad = 0;
+    if (n <= UPLOAD_SHORT) bad = upload_short(l, n, a.c.D, sig);
+    else {
+        if (n <= 32) ref_insertion_sort(l, (int)n, LitLess());
+        else std_sort_replica(l, l + n, LitLess());
+        for (u32 k = 0; k < n; k++) {
+            const u32 lit = l[k];
+            bad |= lit < 2 || lit >= a.c.D || (k && ABS(lit) == ABS(l[k - 1]));
+            sig |= MAPHASH(lit);
+        }
     }
+    if (bad) { set_err(a.c, ERR_INPUT); return; }
     Hdr h;
     h.start = (u32)s;
     h.size = n;
@@ -177,29 +212,48 @@ HD void k_count_formula(const FormulaCountArgs& a, u32 i) {
 }
 
 #if SIGMA_CUDA
-// Same count; lanes of a warp that share a formula (a formula's clauses are
-// mostly adjacent) add once.
-__global__ void count_formula_k(FormulaCountArgs a, u32 n) {
+// Same count. A formula's clauses are mostly adjacent, so a warp takes a stretch of
+// consecutive clauses and adds only where the formula changes: an atomic per step of 32
+// clauses queued 900k of them on 384 words (250 us for 14M clauses of 384 formulas, 167 so).
+__global__ void __launch_bounds__(256) count_formula_k(FormulaCountArgs a, u32 n) {
     const u32 lane = threadIdx.x & 31u;
-    for (u32 base = blockIdx.x * blockDim.x; base < n; base += blockDim.x * gridDim.x) {
-        const u32 i = base + threadIdx.x;
-        u32 f = NONE, cls = 0, lits = 0;
+    const u32 warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    const u32 steps = ((n + 31u) / 32u + nwarps - 1u) / nwarps;  // per warp
+    const u64 first = (u64)warp * steps * 32u;
+    u32 cur = NONE;          // the formula being summed (the same in every lane)
+    u32 cls = 0, lits = 0;   // this lane's share
+    auto flush = [&]() {
+        const u32 tc = __reduce_add_sync(kFull, cls), tl = __reduce_add_sync(kFull, lits);
+        if (lane == 0 && tc) {
+            atomicAdd((unsigned long long*)&a.f_cls[cur], (unsigned long long)tc);
+            atomicAdd((unsigned long long*)&a.f_lits[cur], (unsigned long long)tl);
+        }
+        cls = lits = 0;
+    };
+    for (u32 s = 0; s < steps; s++) {
+        const u64 i = first + (u64)s * 32u + lane;
+        u32 f = NONE, sz = 0;
         if (i < n) {
             const Hdr h = a.c.hdr[i];
             if (!h_deleted(h.flags)) {
                 f = a.c.var_fid[ABS(a.c.lits[h.start])];
-                cls = 1;
-                lits = h.size;
+                sz = h.size;
             }
         }
-        const u32 peers = __match_any_sync(0xffffffffu, f);
-        cls = __reduce_add_sync(peers, cls);
-        lits = __reduce_add_sync(peers, lits);
-        if (f != NONE && lane == (u32)(__ffs(peers) - 1)) {
-            atomicAdd((unsigned long long*)&a.f_cls[f], (unsigned long long)cls);
-            atomicAdd((unsigned long long*)&a.f_lits[f], (unsigned long long)lits);
+        u32 left = __ballot_sync(kFull, f != NONE);
+        while (left) {
+            const u32 g = __shfl_sync(kFull, f, __ffs(left) - 1);
+            if (g != cur) {
+                flush();
+                cur = g;
+            }
+            const bool mine = f == g;
+            cls += mine;
+            lits += mine ? sz : 0u;
+            left &= ~__ballot_sync(kFull, mine);
         }
     }
+    flush();
 }
 
 // Same counts with a warp/block reduction and one pair of atomics per block.
@@ -228,34 +282,42 @@ __global__ void count_live_k(const Hdr* __restrict__ hdr, u32 n, u64* out) {
 
 // ---------------------------------------------------------------- compaction
 // shrinkSimp (src/cpu/simplify.cpp:234-245; GPU: recycle.cu:30-97): drop deleted
-// clauses, keep order. Two exclusive scans (kept clauses, kept literals) give the
-// new id and the new literal start of every survivor.
-struct GcArgs {
+// clauses, keep order. One scan over the clauses gives every survivor its new id (the
+// sum's high word) and its new literal start (the low word: the literals of a store stay
+// below 2^32), and moves it there in the same pass. (Flags, two scans and the move were
+// four passes: 3.7 ms for the compactions of a round over 80M community clauses,
+// 2.6 in one; 300k clauses 127 and 78 us.)
+struct GcMove {
     Ctx c;
-    const u32* keep_scan;    // exclusive scan of keep flags
-    const u64* lit_scan;     // exclusive scan of kept sizes
     Hdr* new_hdr;
     u32* new_lits;
     u32* new_stamp;  // the clause stamps move with the headers
+    typedef ScanNone State;
+    static constexpr int kItems = 4;
+    static HD u32 clauses(u64 sum) { return (u32)(sum >> 32); }
+    static HD u64 lits(u64 sum) { return sum & 0xFFFFFFFFull; }
+    HD u64 value(size_t i, State&) const {
+        const Hdr h = c.hdr[i];
+        return h_deleted(h.flags) ? 0ull : (1ull << 32) + h.size;
+    }
+    HD void done(const State&) const {}
+    HD void put(size_t i, u64 own, u64 at) const {
+        if (!own) return;
+        const u32 id = clauses(at);
+        Hdr h = c.hdr[i];
+        const u32* src = c.lits + h.start;
+        h.start = (u32)lits(at);
+        u32* dst = new_lits + h.start;
+        new_hdr[id] = h;
+        if (c.cstamp) new_stamp[id] = c.cstamp[i];
+        for (u32 k0 = 0; k0 < h.size; k0 += 4) {  // four loads in flight
+            u32 l[4];
+#pragma unroll
+            for (u32 j = 0; j < 4; j++) if (k0 + j < h.size) l[j] = src[k0 + j];
+#pragma unroll
+            for (u32 j = 0; j < 4; j++) if (k0 + j < h.size) dst[k0 + j] = l[j];
+        }
+    }
 };
-HD void k_gc_flags(const Ctx& c, u32* keep, u64* sizes, u32 i) {
-    const Hdr h = c.hdr[i];
-    const bool k = !h_deleted(h.flags);
-    keep[i] = k ? 1u : 0u;
-    sizes[i] = k ? (u64)h.size : 0ull;
-}
-HD void k_gc_move(const GcArgs& a, u32 i) {
-    const Hdr h = a.c.hdr[i];
-    if (h_deleted(h.flags)) return;
-    const u32 id = a.keep_scan[i];
-    const u64 st = a.lit_scan[i];
-    Hdr nh = h;
-    nh.start = (u32)st;
-    a.new_hdr[id] = nh;
-    if (a.c.cstamp) a.new_stamp[id] = a.c.cstamp[i];
-    const u32* src = a.c.lits + h.start;
-    u32* dst = a.new_lits + st;
-    for (u32 k = 0; k < h.size; k++) dst[k] = src[k];
-}
 
 }  // namespace sigma

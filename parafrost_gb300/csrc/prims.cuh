@@ -12,12 +12,16 @@
 
 namespace sigma {
 
-// The plain scan of an array (scan1_k's value and put).
+// The plain scan of an array (scan1_k's value and put; no state per thread).
+struct ScanNone {};
 template <class Tin, class T>
 struct ScanArray {
     const Tin* in;
     T* out;
-    HD T value(size_t i) const { return (T)in[i]; }
+    typedef ScanNone State;
+    static constexpr int kItems = 16;
+    HD T value(size_t i, State&) const { return (T)in[i]; }
+    HD void done(const State&) const {}
     HD void put(size_t i, T, T prefix) const { out[i] = prefix; }
 };
 
@@ -143,44 +147,47 @@ struct Scan1State {
     u32* err;
 };
 
-// A tile is kScan1Items consecutive items per thread: read once from memory in
+// A tile is F::kItems consecutive items per thread (16 for plain arrays, fewer where put
+// has more to do, so that middle-sized scans still have a block for every SM): read once from memory in
 // coalesced order into shared memory, scanned per thread in registers, combined
 // across the block by one warp scan of the thread sums, and written back in
 // coalesced order. Shared-memory positions are padded (one slot per 32) so the
 // per-thread runs of consecutive items do not fall on one bank.
-constexpr int kScan1Items = 16;
-constexpr int kScan1Tile = kScanThreads * kScan1Items;
 __device__ __forceinline__ int scan1_pad(int i) { return i + (i >> 5); }
 
 //
-// The scanned values come from f.value(i) and go to f.put(i, value, prefix), so a pass
-// that selects, ranks and writes items is one launch.
+// The scanned values come from f.value(i, state) and go to f.put(i, value, prefix), so a
+// pass that selects, ranks and writes items is one launch; a thread's state over its
+// values ends in f.done(state), called by whole warps.
 template <class T, class F>
 __global__ void __launch_bounds__(kScanThreads) scan1_k(F f, size_t n, T* total, Scan1State st, u32 base, u32 epoch) {
-    __shared__ T items[kScan1Tile + kScan1Tile / 32];
+    constexpr int kItems = F::kItems, kTile = kScanThreads * kItems;
+    __shared__ T items[kTile + kTile / 32];
     __shared__ T ws[kScanThreads / 32];
     __shared__ u32 tile_s;
     __shared__ T carry_s;
     if (threadIdx.x == 0) tile_s = atomicAdd(st.counter, 1u) - base;
     __syncthreads();
     const u32 tile = tile_s;
-    const size_t nb = (n + kScan1Tile - 1) / kScan1Tile;
-    const size_t t0 = (size_t)tile * kScan1Tile;
+    const size_t nb = (n + kTile - 1) / kTile;
+    const size_t t0 = (size_t)tile * kTile;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    T own[kScan1Items];
+    T own[kItems];
+    typename F::State state{};
 #pragma unroll
-    for (int k = 0; k < kScan1Items; k++) {
+    for (int k = 0; k < kItems; k++) {
         const int j = k * kScanThreads + threadIdx.x;
         const size_t i = t0 + (size_t)j;
-        own[k] = i < n ? f.value(i) : T(0);
+        own[k] = i < n ? f.value(i, state) : T(0);
         items[scan1_pad(j)] = own[k];
     }
+    f.done(state);
     __syncthreads();
-    // this thread's run: items [threadIdx.x * kScan1Items, +kScan1Items)
+    // this thread's run: items [threadIdx.x * kItems, +kItems)
     T run = 0;
-    const int r0 = threadIdx.x * kScan1Items;
+    const int r0 = threadIdx.x * kItems;
 #pragma unroll
-    for (int k = 0; k < kScan1Items; k++) run += items[scan1_pad(r0 + k)];
+    for (int k = 0; k < kItems; k++) run += items[scan1_pad(r0 + k)];
     const T incl = warp_incl_scan(run);
     if (lane == 31) ws[warp] = incl;
     __syncthreads();
@@ -242,7 +249,7 @@ __global__ void __launch_bounds__(kScanThreads) scan1_k(F f, size_t n, T* total,
     // exclusive prefixes of this thread's run, in place
     T acc = carry_s + ws[warp] + incl - run;
 #pragma unroll
-    for (int k = 0; k < kScan1Items; k++) {
+    for (int k = 0; k < kItems; k++) {
         const int q = scan1_pad(r0 + k);
         const T v = items[q];
         items[q] = acc;
@@ -250,14 +257,15 @@ __global__ void __launch_bounds__(kScanThreads) scan1_k(F f, size_t n, T* total,
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kScan1Items; k++) {
+    for (int k = 0; k < kItems; k++) {
         const int j = k * kScanThreads + threadIdx.x;
         const size_t i = t0 + (size_t)j;
         if (i < n) f.put(i, own[k], items[scan1_pad(j)]);
     }
 }
 
-inline size_t scan1_tiles(size_t n) { return (n + kScan1Tile - 1) / kScan1Tile; }
+template <class F>
+size_t scan1_tiles(size_t n) { return (n + kScanThreads * F::kItems - 1) / (kScanThreads * F::kItems); }
 
 // ---------------------------------------------------------------- radix sort
 // Stable LSD radix sort of pairs, 8 bits a pass. One launch counts the digits of every

@@ -40,8 +40,6 @@ struct FHist { Ctx c; HD void operator()(u32 i) const { k_hist_clause(c, i); } }
 struct FScatter { Ctx c; HD void operator()(u32 i) const { k_scatter_clause(c, i); } };
 struct FOccursCl { Ctx c; HD void operator()(u32 i) const { k_occurs_clause(c, i); } };
 struct FCount { CountArgs a; HD void operator()(u32 i) const { k_count_clause(a, i); } };
-struct FGcFlags { Ctx c; u32* keep; u64* sizes; HD void operator()(u32 i) const { k_gc_flags(c, keep, sizes, i); } };
-struct FGcMove { GcArgs a; HD void operator()(u32 i) const { k_gc_move(a, i); } };
 struct FPropLists { PropArgs a; HD void operator()(u32 i) const { k_prop_lists(a, i); } };
 struct FPropClause { PropArgs a; HD void operator()(u32 i) const { k_prop_clause(a, i); } };
 struct FPropSweep { PropArgs a; HD void operator()(u32 i) const { k_prop_sweep(a, i); } };
@@ -570,10 +568,10 @@ struct pf_sigma_ctx {
     void scan1_launch(const Tin* in, T* out, size_t n, T* total) {
         scan_each(ScanArray<Tin, T>{in, out}, n, total);
     }
-    // f.put(i, f.value(i), sum of the values before i) for i in [0, n)
+    // f.put(i, value, sum of the values before i) for i in [0, n), value = f.value(i, state)
     template <class T, class F>
     void scan_each(const F& f, size_t n, T* total) {
-        const size_t tiles = scan1_tiles(n);
+        const size_t tiles = scan1_tiles<F>(n);
         if (!scan1_ctl.p || scan1_base > 0x7FFFFFFFu || scan1_epoch >= 0x3FFFFFFFu) {
             scan1_ctl.reserve(rt, 4);
             rt.zero(scan1_ctl.p, 16);
@@ -606,10 +604,13 @@ struct pf_sigma_ctx {
     template <class T, class F>
     void scan_each(const F& f, size_t n, T* total) {
         T t = 0;
+        typename F::State state{};
+        std::vector<T> own(n);
+        for (size_t i = 0; i < n; i++) own[i] = f.value(i, state);
+        f.done(state);
         for (size_t i = 0; i < n; i++) {
-            const T v = f.value(i);
-            f.put(i, v, t);
-            t += v;
+            f.put(i, own[i], t);
+            t += own[i];
         }
         *total = t;
     }
@@ -1610,28 +1611,18 @@ struct pf_sigma_ctx {
             compact = true;
             return;
         }
-        big32a.reserve(rt, (size_t)ncls + 1);
-        big32b.reserve(rt, (size_t)ncls + 1);
-        big64a.reserve(rt, (size_t)ncls + 1);
-        big64b.reserve(rt, (size_t)ncls + 1);
-        Ctx c = view();
-        rt.each(FGcFlags{c, big32a.p, big64a.p}, ncls);
-        scan_to(big32a.p, big32b.p, ncls, 0);
-        scan_to(big64a.p, big64b.p, ncls, 1);
-        u32 keep = (u32)n_cls_after;
-        u64 keep_lits = (u64)n_lits_after;
-        if (counted) {
-            slots = ReadSlots{};
-        } else {
-            read_slots_checked();
-            keep = (u32)hr[0];
-            keep_lits = hr[1];
-        }
         hdr2.reserve(rt, hdr.n);
         cstamp2.reserve(rt, hdr.n);
-        lits2.reserve(rt, std::max<size_t>(lits.n, (size_t)keep_lits + 16));
-        GcArgs g{c, big32b.p, big64b.p, hdr2.p, lits2.p, cstamp2.p};
-        rt.each(FGcMove{g}, ncls);
+        lits2.reserve(rt, lits.n);
+        scan_each(GcMove{view(), hdr2.p, lits2.p, cstamp2.p}, ncls, hslot(0));
+        u32 keep = (u32)n_cls_after;
+        u64 keep_lits = (u64)n_lits_after;
+        if (!counted) {
+            word64_to(hslot(0), 0);
+            read_slots_checked();
+            keep = GcMove::clauses(hr[0]);
+            keep_lits = GcMove::lits(hr[0]);
+        }
         std::swap(hdr, hdr2);
         std::swap(cstamp, cstamp2);
         std::swap(lits, lits2);
