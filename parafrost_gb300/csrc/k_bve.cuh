@@ -473,10 +473,4 @@ __global__ void __launch_bounds__(256, 6) bve_write_warp_k(BveArgs a, const u32*
 }
 #endif
 
-// Per-variable scratch words for the AND/OR fan-in list.
-HD void k_bve_scratch_need(const Ctx& c, const u32* pvs, u64* need, u32 k) {
-    const u32 p = V2L(pvs[k]);
-    need[k] = (u64)c.ot_size[p] + c.ot_size[NEG(p)] + 2;
-}
-
 }  // namespace sigma

@@ -167,7 +167,8 @@ HD void sub_update_list(const Ctx& c, u32 l) {
 
 // Whether SUB on this variable can produce a unit: some binary (x u) in the
 // positive list next to a binary (-x u) in the negative list. Counts producers in
-// *flag and, with prod, sets prod[k] (cleared first).
+// *flag and, with prod, sets prod[k] (cleared first). The lists are sorted by size, so
+// the binaries are looked for at their fronts only.
 HD void k_sub_unit_possible(const SubArgs& a, u32* flag, u32* prod, u32 k) {
     const Ctx& c = a.c;
     const u32 v = a.pvs[k];
@@ -177,11 +178,13 @@ HD void k_sub_unit_possible(const SubArgs& a, u32* flag, u32* prod, u32 k) {
     const u32 po = c.ot_off[p], ps = c.ot_size[p], no = c.ot_off[n], ns = c.ot_size[n];
     for (u32 i = 0; i < ps; i++) {
         const Hdr hi = c.hdr[c.ot_refs[po + i]];
+        if (hi.size > 2) break;
         if (hi.size != 2 || h_deleted(hi.flags)) continue;
         const u32* li = c.lits + hi.start;
         const u32 ui = li[0] == p ? li[1] : li[0];
         for (u32 j = 0; j < ns; j++) {
             const Hdr hj = c.hdr[c.ot_refs[no + j]];
+            if (hj.size > 2) break;
             if (hj.size != 2 || h_deleted(hj.flags)) continue;
             const u32* lj = c.lits + hj.start;
             const u32 uj = lj[0] == n ? lj[1] : lj[0];

@@ -63,7 +63,9 @@ struct FProofClause {
         if (!h_deleted(h.flags) && h.size > 1) proof_line(c, c.lits + h.start, h.size);
     }
 };
-struct FSortList { SortArgs a; HD void operator()(u32 i) const { k_sort_list(a, i); } };
+#if !SIGMA_CUDA
+struct FSortPv { SortArgs a; HD void operator()(u32 k) const { k_sort_pv(a, k); } };
+#endif
 struct FSubPossible { SubArgs a; u32* flag; u32* prod; HD void operator()(u32 i) const { k_sub_unit_possible(a, flag, prod, i); } };
 struct FSubNeed {
     Ctx c; const u32* pvs; const uint8_t* only; u32* ent; u64* words;
@@ -106,7 +108,6 @@ struct FSubCommitItem {
 };
 struct FSubCommitClear { Ctx c; const u32* lits; HD void operator()(u32 q) const { k_sub_commit_clear(c, lits, q); } };
 struct FSubAssign { Ctx c; const U2* units; HD void operator()(u32 i) const { enqueue_unit(c, units[i].y); } };
-struct FBveNeed { Ctx c; const u32* pvs; u64* need; HD void operator()(u32 i) const { k_bve_scratch_need(c, pvs, need, i); } };
 struct FBveWarp { BveArgs a; HD void operator()(u32 i) const { k_bve_warp(a, i); } };
 struct FBveWrite { BveArgs a; HD void operator()(u32 i) const { k_bve_write(a, i); } };
 struct FBceCountWarp { BceArgs a; HD void operator()(u32 i) const { bce_count_warp(a, i); } };
@@ -137,18 +138,6 @@ struct Perm {
     F f;
     const u32* perm;
     HD void operator()(u32 i) const { f(perm[i]); }
-};
-// Work-order key of elected variable k: descending clause count.
-// Elected variables from n_first on (a batch's stopping formulas) come after the
-// others; clause counts from 127 up share the first place (one 8-bit radix pass).
-struct FPvKey {
-    Ctx c; const u32* pvs; u32* key; u32* val; u32 n_first;
-    HD void operator()(u32 k) const {
-        const u32 p = V2L(pvs[k]);
-        const u32 occ = c.ot_size[p] + c.ot_size[p + 1];
-        key[k] = (k >= n_first ? 0x80u : 0u) | (0x7Fu - (occ < 0x7Fu ? occ : 0x7Fu));
-        val[k] = k;
-    }
 };
 struct FVarFid { u32* var_fid; const u32* f_var; u32 nf; HD void operator()(u32 v) const { k_var_fid(var_fid, f_var, nf, v); } };
 struct FCountFormula { FormulaCountArgs a; HD void operator()(u32 i) const { k_count_formula(a, i); } };
@@ -1139,14 +1128,23 @@ struct pf_sigma_ctx {
 
     void sort_ot() {
         rt.zero(ws_slots.p, kSpreadSlots * 8);
-        SortArgs a{view(), pvs.p, ws_slots.p};
-        rt.each(FSortList{a}, 2 * npvs);
         // work order of the per-variable kernels: most clauses first (longest
         // processing time first), so similar variables share a warp and the longest
         // ones do not start last. Results still go to each variable's elected rank.
         pv_perm.reserve(rt, nvars + 1);
         pv_key.reserve(rt, nvars + 1);
-        rt.each(FPvKey{view(), pvs.p, pv_key.p, pv_perm.p, n_go}, npvs);
+        big64a.reserve(rt, (size_t)npvs + 1);  // BVE scratch words, scanned by pv_prepare
+        SortArgs a{view(), pvs.p, ws_slots.p, npvs, n_go, pv_key.p, pv_perm.p, big64a.p};
+#if SIGMA_CUDA
+        if (npvs) {
+            const int smem = SORT_WARPS * (int)sizeof(SortStage);
+            rt.launches++;
+            sort_lists_k<<<rt.grid((npvs + 15) / 16 * 32), SORT_WARPS * 32, smem, rt.stream>>>(a);
+            ck(cudaGetLastError(), "launch");
+        }
+#else
+        rt.each(FSortPv{a}, npvs);
+#endif
         sort_pairs(pv_key.p, pv_perm.p, order_k2.p, order_v2.p, npvs, 8);
     }
 
@@ -1178,8 +1176,6 @@ struct pf_sigma_ctx {
         }
         if (n && opt.ve) {
             ve_scr_off.reserve(rt, n + 1);
-            big64a.reserve(rt, n + 1);
-            rt.each(FBveNeed{view(), pvs.p, big64a.p}, n);
             scan_to(big64a.p, ve_scr_off.p, n, 0);
         }
         read_slots_checked();
