@@ -383,7 +383,6 @@ __device__ void bve_write_warp(const BveArgs& a, u32 k) {
     const Ctx& c = a.c;
     const u32 lane = threadIdx.x & 31u;
     const uint8_t type = a.type[k];
-    if (type == VE_KEEP) return;
     if (type == VE_EQU || !a.ncls[k]) {
         if (lane == 0) k_bve_write(a, k);
         __syncwarp();
@@ -467,7 +466,14 @@ __global__ void __launch_bounds__(256, 6) bve_write_warp_k(BveArgs a, const u32*
         j0 = __shfl_sync(0xffffffffu, j0, 0);
         if (j0 >= npos) break;
         const u32 j1 = j0 + chunk < npos ? j0 + chunk : npos;
-        for (u32 j = j0; j < j1; j++) bve_write_warp(a, perm[j]);
+        // the variables of a grab that are kept cost one load by one lane each
+        const u32 kq = lane < j1 - j0 ? perm[j0 + lane] : 0u;
+        u32 todo = __ballot_sync(kFull, lane < j1 - j0 && a.type[kq] != VE_KEEP);
+        while (todo) {
+            const int q = __ffs(todo) - 1;
+            todo &= todo - 1;
+            bve_write_warp(a, __shfl_sync(kFull, kq, q));
+        }
         chunk = warp_chunk(npos - j1);
     }
 }

@@ -114,7 +114,12 @@ struct FBceCountWarp { BceArgs a; HD void operator()(u32 i) const { bce_count_wa
 struct FBceWrite { BceArgs a; HD void operator()(u32 i) const { k_bce_write(a, i); } };
 struct FEre { EreArgs a; HD void operator()(u32 i) const { k_ere_pv(a, i); } };
 struct FEreCount { EreArgs a; const u32* perm; u64* cnt; HD void operator()(u32 q) const { k_ere_count(a, perm, cnt, q); } };
-struct FErePair { EreArgs a; const u32* perm; const u64* off; u32 n; HD void operator()(u32 i) const { k_ere_pair(a, perm, off, n, i); } };
+#if !SIGMA_CUDA
+struct FErePair {
+    EreArgs a; const u32* perm; const u64* off; u32 n;
+    HD void operator()(u32 i) const { k_ere_pair(a, perm, off, upper_segment(off, n, (u64)i), i); }
+};
+#endif
 struct FEreResolve { EreArgs a; HD void operator()(u32 i) const { k_ere_resolve(a, i); } };
 struct FEreFix { EreArgs a; const u64* keys; u32 n; HD void operator()() const { ere_fixup(a, keys, n); } };
 // Sort keys of the ERE losers: loser order[i]'s low key word (hi = false; order[i] =
@@ -1555,8 +1560,18 @@ struct pf_sigma_ctx {
         big64b.reserve(rt, (size_t)perm_n + 1);
         rt.each(FEreCount{a, pv_perm.p + perm_off, big64a.p}, perm_n);
         const u64 pairs = scan64(big64a.p, big64b.p, perm_n);
-        if (pairs < 0xFFFFFFF0ull) rt.each(FErePair{a, pv_perm.p + perm_off, big64b.p, perm_n}, (u32)pairs);
-        else pv_each(FEre{a});
+        if (pairs >= 0xFFFFFFF0ull) {
+            pv_each(FEre{a});
+        } else if (pairs) {
+#if SIGMA_CUDA
+            rt.launches++;
+            ere_pair_k<<<rt.grid((u32)pairs), 256, 0, rt.stream>>>(a, pv_perm.p + perm_off, big64b.p, perm_n,
+                                                                   (u32)pairs);
+            ck(cudaGetLastError(), "launch");
+#else
+            rt.each(FErePair{a, pv_perm.p + perm_off, big64b.p, perm_n}, (u32)pairs);
+#endif
+        }
         check();
         const u32 nrec = read_u32(counters.p + 7);
         rt.each(FEreResolve{a}, nrec);
