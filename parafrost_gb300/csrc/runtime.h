@@ -88,6 +88,7 @@ __global__ void read_slots_k(ReadSlots s, u64* out) {
 struct Runtime {
     Stream stream = nullptr;
     int sms = 152;
+    bool host_reads = false;  // kernels can read any host memory (through the host's page tables)
     size_t bytes_live = 0;
     size_t budget = 0;  // 0 = no limit
     unsigned launches = 0;
@@ -107,6 +108,10 @@ struct Runtime {
         int dev = 0;
         ck(cudaGetDevice(&dev), "cudaGetDevice");
         ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr");
+        int pageable = 0, tables = 0;
+        ck(cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev), "attr");
+        ck(cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev), "attr");
+        host_reads = pageable && tables;
         ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "stream");
 #endif
     }

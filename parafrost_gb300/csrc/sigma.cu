@@ -348,6 +348,9 @@ struct pf_sigma_ctx {
     DBuf<u64> up_off;           // offsets of an upload from host buffers
     DBuf<u64> up_first, up_base, up_cls;  // per formula of a batch upload
     DBuf<u32> up_nv;
+#if SIGMA_CUDA
+    DBuf<UploadPiece> up_pieces;
+#endif
     // batch results and model extension: records, units and values in formula order
     DBuf<u32> rs_flag, rs_scan, rs_start, rs_key, rs_val, rs_k2, rs_v2, rs_out, rs_first;
     DBuf<u64> rs_words, rs_size, rs_off, rs_fsum, rs_pfirst;
@@ -2297,6 +2300,38 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
             // each formula's literals and offsets straight to their place; offsets
             // are rebased on the device
             doff.reserve(rt, num_clauses + 1);
+#if SIGMA_CUDA
+            bool in_place = rt.host_reads;  // (a kernel's loads need aligned words, a copy does not)
+            for (u32 f = 0; f < batch->nf; f++)
+                in_place &= !((uintptr_t)batch->part_lits[f] & 3u) && !((uintptr_t)batch->part_offsets[f] & 7u);
+            if (in_place) {
+                std::vector<UploadPiece> pieces;
+                u64 at = 0;
+                for (u32 f = 0; f < batch->nf; f++) {
+                    const u64 cb = batch->clause_begin[f], nc = batch->clause_begin[f + 1] - cb;
+                    const u64* o = batch->part_offsets[f];
+                    const u64 len = o[nc] - o[0];
+                    for (u64 i = 0; i < len; i += PART_WORDS)
+                        pieces.push_back({batch->part_lits[f] + o[0] + i, at + i, 0,
+                                          (u32)std::min<u64>(len - i, PART_WORDS), 0u});
+                    for (u64 i = 0; i < nc; i += PART_WORDS)
+                        pieces.push_back({o + i, cb + i, at - o[0], (u32)std::min<u64>(nc - i, PART_WORDS), 1u});
+                    at += len;
+                }
+                c.write_u64(doff.p + num_clauses, at);
+                c.up_pieces.reserve(rt, pieces.size() + 1);
+                rt.h2d(c.up_pieces.p, pieces.data(), pieces.size() * sizeof(UploadPiece));
+                if (!pieces.empty()) {
+                    rt.launches++;
+                    const u32 np = (u32)pieces.size();
+                    upload_pieces_k<<<std::min(np, (u32)rt.sms * 8u), 256, 0, rt.stream>>>(c.up_pieces.p, np, c.lits.p,
+                                                                                           doff.p);
+                    ck(cudaGetLastError(), "launch");
+                }
+                rt.sync();
+            } else
+#endif
+            {
             std::vector<u64> first(batch->nf), base(batch->nf);
             u64 at = 0;
             for (u32 f = 0; f < batch->nf; f++) {
@@ -2319,6 +2354,7 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
             rt.h2d(dcb.p, batch->clause_begin, (batch->nf + 1) * 8);
             if (num_clauses) rt.each(FRebase{doff.p, dcb.p, dfirst.p, dbase.p, batch->nf}, (u32)num_clauses);
             rt.sync();  // the host arrays of this block are done with
+            }
             off_ptr = doff.p;
         } else if (device) {
             rt.d2d(c.lits.p, lits + off0, L * 4);
