@@ -121,7 +121,10 @@ struct FErePair {
 };
 #endif
 struct FEreResolve { EreArgs a; HD void operator()(u32 i) const { k_ere_resolve(a, i); } };
-struct FEreFix { EreArgs a; const u64* keys; u32 n; HD void operator()() const { ere_fixup(a, keys, n); } };
+struct FEreFix {
+    EreArgs a; const u64* keys; const u32* target; u32 n;
+    HD void operator()(u32 q) const { ere_fixup(a, keys, target, n, q); }
+};
 // Sort keys of the ERE losers: loser order[i]'s low key word (hi = false; order[i] =
 // i set first) or high key word (hi = true), and the keys in sorted order.
 struct FEreLoserKey {
@@ -132,10 +135,15 @@ struct FEreLoserKey {
         out[i] = hi ? (u32)(k >> 32) : (u32)k;
     }
 };
+struct FEreLoserTarget {
+    const u32* target; const u32* losers; const u32* order; u32* out;
+    HD void operator()(u32 i) const { out[i] = target[losers[order[i]]]; }
+};
 struct FEreLoserGather {
     const u64* key; const u32* losers; const u32* order; u64* out;
     HD void operator()(u32 i) const { out[i] = key[losers[order[i]]]; }
 };
+struct FIota { u32* p; HD void operator()(u32 i) const { p[i] = i; } };
 struct FEreSeq { EreArgs a; HD void operator()() const { ere_sequential(a); } };
 // Item i of a permuted launch runs f(perm[i]).
 template <class F>
@@ -1532,19 +1540,17 @@ struct pf_sigma_ctx {
         if (!opt.ere || !npvs) return;
         proof_reserve(nlits_used + ncls + 16);  // a deletion line per clause at most
         if (opt.ere_max > 65535) throw std::runtime_error("eremax above 65535 is not supported");
-        EreArgs a;
+        EreArgs a{};
         a.c = view();
         a.pvs = pvs.p;
         a.npvs = npvs;
         a.ere_max = (u32)opt.ere_max;
         a.ere_clause_max = opt.ere_clause_max;
-        if (has_learnt) {
-            rt.one(FEreSeq{a});
-            rt.sync();
-            return;
+        a.in_order = has_learnt;
+        if (!has_learnt) {
+            ere_claim.reserve(rt, hdr.n);
+            rt.zero(ere_claim.p, (size_t)ncls * 8, 0xFF);
         }
-        ere_claim.reserve(rt, hdr.n);
-        rt.zero(ere_claim.p, (size_t)ncls * 8, 0xFF);
         const size_t cap_rec = (size_t)ncls + (1u << 20);
         ere_target.reserve(rt, cap_rec);
         ere_key.reserve(rt, cap_rec);
@@ -1577,11 +1583,19 @@ struct pf_sigma_ctx {
         }
         check();
         const u32 nrec = read_u32(counters.p + 7);
-        rt.each(FEreResolve{a}, nrec);
-        const u32 nl = read_u32(counters.p + 8);
+        u32 nl = nrec;
+        if (!has_learnt) {
+            rt.each(FEreResolve{a}, nrec);
+            nl = read_u32(counters.p + 8);
+        } else if (nrec > cap_rec) {
+            rt.one(FEreSeq{a});
+            return;
+        } else {
+            rt.each(FIota{ere_losers.p}, nrec);
+        }
         if (nl) {
-            // the losers' keys in ascending order, sorted on the device: by the low
-            // word (pair), then stably by the high word (elected rank)
+            // the losers by first target and key, sorted on the device: by the key's low
+            // word (pair), then stably by its high word (elected rank) and the target
             big32a.reserve(rt, (size_t)nl + 1);
             big32b.reserve(rt, (size_t)nl + 1);
             work.reserve(rt, 2 * (size_t)nl + 2);
@@ -1591,8 +1605,10 @@ struct pf_sigma_ctx {
             rt.each(FEreLoserKey{ere_key.p, ere_losers.p, big32b.p, big32a.p, true}, nl);
             const int rb = key_bits(npvs);
             sort_pairs(big32a.p, big32b.p, work.p, work.p + nl + 1, nl, rb);
+            rt.each(FEreLoserTarget{ere_target.p, ere_losers.p, big32b.p, big32a.p}, nl);
+            sort_pairs(big32a.p, big32b.p, work.p, work.p + nl + 1, nl, key_bits(ncls));
             rt.each(FEreLoserGather{ere_key.p, ere_losers.p, big32b.p, big64b.p}, nl);
-            rt.one(FEreFix{a, big64b.p, nl});
+            rt.each(FEreFix{a, big64b.p, big32a.p, nl}, nl);
         }
     }
 
