@@ -329,29 +329,83 @@ __global__ void __launch_bounds__(256) mis_rec_warp_k(LcveArgs a, Q4* rec) {
     if (lane == 0 && sum) atomicAdd((unsigned long long*)(a.ws_bytes + (blockIdx.x & (kSpreadSlots - 1u))),
                                     (unsigned long long)sum);
 }
+
+// The same with a thread a clause, four literals at a time: their loads, then their words'
+// loads, are in flight together, and the next clause's header. A warp of the kernel above
+// waits for both at every 32 literals, which more warps hide on a large store but nothing
+// hides on one that does not fill the chip. Clause records of a round, warps and threads:
+// 200 variables 42 and 16 us, 43k clauses 89 and 19, 1M mixed 134 and 98, a 6.8M-clause AIG 362
+// and 384, 14M clauses of 384 formulas 1.11 and 1.25 ms, 80M community clauses 3.5 and 4.2:
+// threads below MIS_REC_WARPS clauses.
+constexpr u32 MIS_REC_WARPS = 1u << 20;
+__global__ void __launch_bounds__(256) mis_rec_k(LcveArgs a, Q4* rec) {
+    const u32 lane = threadIdx.x & 31u;
+    const u32 step = gridDim.x * blockDim.x;
+    u64 sum = 0;
+    u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    Hdr h{};
+    if (i < a.c.ncls) h = hdr_ro(&a.c.hdr[i]);
+    for (; i < a.c.ncls;) {
+        const Hdr cur = h;
+        const u32 at = i;
+        i = a.c.ncls - i > step ? i + step : a.c.ncls;
+        if (i < a.c.ncls) h = hdr_ro(&a.c.hdr[i]);
+        const u32* l = a.c.lits + cur.start;
+        const bool dead = h_deleted(cur.flags);
+        u32 ng = 0, m = MIS_NO_RANK;
+        Q4 q;
+        q.x = q.y = q.z = 0u;
+        for (u32 k0 = 0; k0 < cur.size; k0 += 4) {
+            u32 x[4], w[4];
+#pragma unroll
+            for (u32 j = 0; j < 4; j++) x[j] = k0 + j < cur.size ? __ldg(&l[k0 + j]) : 0u;
+#pragma unroll
+            for (u32 j = 0; j < 4; j++) w[j] = k0 + j < cur.size ? ldro(&a.word[ABS(x[j])]) : MIS_NO_RANK;
+            if (!k0) {
+                q.x = x[0];
+                q.y = x[1];
+                q.z = x[2];
+            }
+#pragma unroll
+            for (u32 j = 0; j < 4; j++) {
+                const u32 rk = mis_rank(w[j]);
+                ng += rk != MIS_NO_RANK;
+                m = rk < m ? rk : m;
+            }
+        }
+        q.w = cur.size | (dead ? 0x80000000u : 0u);
+        rec[at] = q;
+        a.cmin[at] = dead ? MIS_NO_RANK : m;
+        sum += (u64)ng * (4ull + (dead ? 0ull : 8ull + 4ull * cur.size));
+    }
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0 && sum) atomicAdd((unsigned long long*)(a.ws_bytes + (blockIdx.x & (kSpreadSlots - 1u))),
+                                    (unsigned long long)sum);
+}
 #endif
 
-// Whether clause cl holds a graph neighbour of v ranked below rv that is not out
-// (decisions are read through to the cache level other SMs write).
-HD bool mis_blocked_in(const LcveArgs& a, u32 v, u32 rv, const MisCl& cl) {
-    if (cl.r0) return cl.q.x < rv;
-    if (cl.deleted()) return false;
+// A graph neighbour of v in clause cl that is ranked below rv and not out (0: none; a
+// first-round clause only says that there is one: NONE). Decisions are read through to the
+// cache level other SMs write.
+HD u32 mis_blocker(const LcveArgs& a, u32 v, u32 rv, const MisCl& cl) {
+    if (cl.r0) return cl.q.x < rv ? NONE : 0u;
+    if (cl.deleted()) return 0;
     const u32 size = cl.size();
     const u32* L = mis_long_lits(a, cl);
     for (u32 k0 = 0; k0 < size; k0 += MIS_CHUNK) {
         u32 w[MIS_CHUNK];
 #pragma unroll
         for (u32 j = 0; j < MIS_CHUNK; j++) w[j] = k0 + j < size ? ABS(mis_lit(cl, L, k0 + j)) : v;
-        bool b = false;
+        u32 b = 0;
 #pragma unroll
         for (u32 j = 0; j < MIS_CHUNK; j++) {
             if (w[j] == v) continue;
             const u32 g = ldcg_hint(&a.word[w[j]], a.pl);
-            b |= mis_rank(g) < rv && mis_dec(g) != MIS_OUT;
+            if (mis_rank(g) < rv && mis_dec(g) != MIS_OUT) b = w[j];
         }
-        if (b) return true;
+        if (b) return b;
     }
-    return false;
+    return 0;
 }
 
 // Vertex v (rank rv) goes in; one whose lists reach the temperatures bounds the election
@@ -374,7 +428,7 @@ HD bool mis_pull_one(const LcveArgs& a, u32 v, u32 wv, bool r0) {
         for (; t < n; t++) {
             MisCl nx = cl;
             if (t + 1 < n) nx = mis_cl(a, ldro_hint(&a.c.ot_refs[t + 1 < np ? op + t + 1 : on + t + 1], a.pf), r0);
-            if (mis_blocked_in(a, v, rv, cl)) {
+            if (mis_blocker(a, v, rv, cl)) {
                 a.resume[v] = t;
                 return false;
             }
@@ -460,7 +514,7 @@ struct MisRounds {
     u32* trace;      // optional: per round [undecided small, big, start ns / 1024]
     u32 trace_cap;   // rounds the trace holds
 };
-constexpr u32 MIS_TRIES = 48;
+constexpr u32 MIS_TRIES = 384;
 
 // Vertices that stay undecided are staged per block in shared memory and copied to the
 // next lists with one reservation per block (a vertex that finds its block's queue full
@@ -532,18 +586,33 @@ DEV void mis_queue_flush(MisBlockQueue& q, const MisFront& f) {
 // them): clauses from `at` on, L at a time in list order, the first blocking one of a
 // step (lowest lane) stops the walk. Returns true when v is decided; a walk that
 // reaches the end puts v in and marks its neighbours out, the lanes sharing the clauses.
-DEV bool mis_try(const LcveArgs& a, u32 v, u32 gm, u32 gbase, u32 sub, u32 L, u32& at, bool r0) {
+// wait: the neighbour that stopped the last try (0 or NONE: none known). Until it is
+// decided only its word and v's own are looked at: one load a try instead of a walk's
+// four dependent ones.
+DEV bool mis_try(const LcveArgs& a, u32 v, u32 gm, u32 gbase, u32 sub, u32 L, u32& at, u32& wait, bool r0) {
     const u32 wv = vload(&a.word[v]);  // the same word for the whole group
+    const bool known = wait && wait != NONE;
+    const u32 ww = known ? vload(&a.word[wait]) : 0u;
     if (mis_dec(wv) != MIS_UNDECIDED) return true;
+    if (known) {
+        if (mis_dec(ww) == MIS_UNDECIDED) return false;
+        if (mis_dec(ww) == MIS_IN) {  // a lower neighbour is in
+            if (sub == 0) atomicOr(&a.word[v], mis_dec_bits(MIS_OUT));
+            return true;
+        }
+    }
     const u32 rv = mis_rank(wv);
     const u32 p = V2L(v), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
     const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
     for (u32 b0 = at; b0 < n; b0 += L) {
         const u32 t = b0 + sub;
-        const bool blk = t < n && mis_blocked_in(a, v, rv, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf), r0));
-        const u32 m = (__ballot_sync(gm, blk) & gm) >> gbase;
+        u32 blk = 0;
+        if (t < n) blk = mis_blocker(a, v, rv, mis_cl(a, ldro_hint(&a.c.ot_refs[t < np ? op + t : on + t], a.pf), r0));
+        const u32 m = (__ballot_sync(gm, blk != 0) & gm) >> gbase;
         if (m) {
-            at = b0 + (u32)(__ffs(m) - 1);
+            const u32 first = (u32)(__ffs(m) - 1);
+            at = b0 + first;
+            wait = __shfl_sync(gm, blk, (int)(gbase + first));
             return false;
         }
     }
@@ -617,10 +686,11 @@ __global__ void __launch_bounds__(256, 6) mis_rounds_k(LcveArgs a0, MisRounds w)
             const bool hb = warp < ub, hs = tid / lu < us;
             const u32 vb = hb ? vload(&pu_b[warp]) : 0u, vs = hs ? vload(&pu_s[tid / lu]) : 0u;
             u32 ab = hb ? vload(&a.resume[vb]) : 0u, as = hs ? vload(&a.resume[vs]) : 0u;
+            u32 nb = 0, ns = 0;  // the neighbours that are waited for
             bool wb = hb, ws = hs;
             for (u32 k = 0; k < MIS_TRIES && __any_sync(kFull, wb || ws); k++) {
-                if (wb) wb = !mis_try(a, vb, kFull, 0, lane, 32, ab, false);  // warp-uniform
-                if (ws) ws = !mis_try(a, vs, gm, gbase, sub, lu, as, false);  // group-uniform
+                if (wb) wb = !mis_try(a, vb, kFull, 0, lane, 32, ab, nb, false);  // warp-uniform
+                if (ws) ws = !mis_try(a, vs, gm, gbase, sub, lu, as, ns, false);  // group-uniform
                 __syncwarp();
             }
             if (wb && lane == 0) {
@@ -632,8 +702,8 @@ __global__ void __launch_bounds__(256, 6) mis_rounds_k(LcveArgs a0, MisRounds w)
         } else {
             for (u32 idx = warp; idx < ub; idx += nwarps) {
                 const u32 v = vload(&pu_b[idx]);
-                u32 at = vload(&a.resume[v]);
-                const bool und = !mis_try(a, v, kFull, 0, lane, 32, at, r0);
+                u32 at = vload(&a.resume[v]), wait = 0;
+                const bool und = !mis_try(a, v, kFull, 0, lane, 32, at, wait, r0);
                 if (und && lane == 0) {
                     a.resume[v] = at;
                     mis_queue_push(qu, fu, true, v);
@@ -676,8 +746,8 @@ __global__ void __launch_bounds__(256, 6) mis_rounds_k(LcveArgs a0, MisRounds w)
                     bool und = false;
                     if (idx < us) {
                         v = vload(&pu_s[idx]);
-                        u32 at = vload(&a.resume[v]);
-                        und = !mis_try(a, v, gm, gbase, sub, lu, at, r0);
+                        u32 at = vload(&a.resume[v]), wait = 0;
+                        und = !mis_try(a, v, gm, gbase, sub, lu, at, wait, r0);
                         if (und && sub == 0) a.resume[v] = at;
                         und = und && sub == 0;
                     }

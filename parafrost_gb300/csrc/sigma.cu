@@ -1061,7 +1061,8 @@ struct pf_sigma_ctx {
 #if SIGMA_CUDA
         if (ncls) {
             rt.launches++;
-            mis_rec_warp_k<<<rt.grid((ncls + 7u) / 8u, 8), 256, 0, rt.stream>>>(a, mis_rec.p);
+            if (ncls < MIS_REC_WARPS) mis_rec_k<<<rt.grid(ncls), 256, 0, rt.stream>>>(a, mis_rec.p);
+            else mis_rec_warp_k<<<rt.grid((ncls + 7u) / 8u, 8), 256, 0, rt.stream>>>(a, mis_rec.p);
             ck(cudaGetLastError(), "launch");
         }
 #else
