@@ -600,7 +600,15 @@ struct PropWaves {
                         // and by the barrier that ends each wave)
 };
 
-__global__ void __launch_bounds__(256, 4) prop_waves_k(PropArgs a, PropWaves w) {
+// Blocks per SM by the store's size: on a small one most waves are small and the barrier
+// between them costs an arrival per block; on a large one sweeps and wide walks want every
+// warp the registers allow. Propagation at 1, 2, 4 and 6 blocks an SM: 1.1M-clause unrolled
+// AIG 3.5, 3.2, 3.7 and 4.9 ms; 120k clauses with learnt ones 186, 201, 268 and 340 us; 8M
+// community clauses 2.48, 1.41, 0.93 and 0.92 ms; 80M 26.1, 14.0, 8.4 and 7.1.
+constexpr u32 PROP_LARGE = 1u << 22;  // clauses
+constexpr int PROP_BLOCKS_SMALL = 2, PROP_BLOCKS_LARGE = 6;
+template <int MinBlocks>
+__global__ void __launch_bounds__(256, MinBlocks) prop_waves_k(PropArgs a, PropWaves w) {
     __shared__ u32 sm[3 * 256];
     __shared__ PropWarp pw[8];
     const u32 tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;

@@ -763,8 +763,12 @@ struct pf_sigma_ctx {
     DBuf<unsigned short> otb_slot;
     bool otb_plan(u32& shift, u32& nb) const {
         if (opt.ot_buckets < 0 || (opt.ot_buckets == 0 && 4ull * (nlits_used + D) < kOtbMinBytes)) return false;
+        // some 2,000 buckets, 4,000 for tables that are much larger than L2 (tables of a
+        // round at 512, 1,024, 2,048 and 4,096: 28M occurrences 1.29, 1.24, 1.23 and 1.61 ms,
+        // 50M of a batch 5.30, 4.57, 4.29 and 5.12, 280M 13.5, 13.5, 13.5 and 13.1)
+        const u64 most = nlits_used >= (1ull << 27) ? 4096 : 2048;
         u32 s = 8;
-        while (s < OTB_MAX_SHIFT && ((u64)D >> s) > 1024) s++;
+        while (s < OTB_MAX_SHIFT && ((u64)D >> s) > most) s++;
         shift = s;
         nb = (u32)(((u64)D + (1ull << s) - 1) >> s);
         return nb <= OTB_MAX_BUCKETS;
@@ -943,10 +947,10 @@ struct pf_sigma_ctx {
             rt.d2d(counters.p + 18, counters.p + 0, 4);  // [18] the trail's end for the first wave
             void* args[] = {&a, &w};
             rt.launches++;
-            // four blocks per SM: most waves of a propagation are small, and the grid
-            // barrier between them costs one arrival per block
-            ck(cudaLaunchCooperativeKernel((const void*)prop_waves_k, dim3(rt.sms * 4), dim3(256), args, 0,
-                                           rt.stream),
+            const bool large = ncls >= PROP_LARGE;
+            const void* kernel = large ? (const void*)prop_waves_k<PROP_BLOCKS_LARGE> : (const void*)prop_waves_k<4>;
+            const u32 per_sm = large ? PROP_BLOCKS_LARGE : PROP_BLOCKS_SMALL;
+            ck(cudaLaunchCooperativeKernel(kernel, dim3(rt.sms * per_sm), dim3(256), args, 0, rt.stream),
                "cooperative launch");
             word_to(counters.p + 26, 0);
             read_slots_checked();
