@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(256, MinBlocks) prop_waves_k(PropArgs a, PropW
     u32 strip_from = a.head;  // trail literals from here on are still to be stripped
     u32 strip_end = a.head;   // while a strip's list parts are left: the literals it took end here
     u32 stamp = a.stamp;      // of the strip
-    u32 wave = 0;
+    u32 wave = 0, walks = 0;
     for (;; wave++) {
         const u32 cur = wave % 3, nxt = (wave + 1) % 3, old = (wave + 2) % 3;
         const u32 tail = vload(w.tail);
@@ -628,7 +628,9 @@ __global__ void __launch_bounds__(256, MinBlocks) prop_waves_k(PropArgs a, PropW
         if (!nq) strip_from = strip_end;
         const bool stripping = strip_end != strip_from;  // the last wave was a strip: nq are its parts
         if (!np && !nq && tail == strip_from && !stripping) break;
-        if (wave >= w.max_waves) {
+        // walks and sweeps count against the bound, one more than level by level: the parts of
+        // a list come a wave after its front
+        if ((np || nq) && !stripping && walks++ > w.max_waves) {
             if (tid == 0) atomicOr(a.c.err, ERR_ITER);
             return;
         }

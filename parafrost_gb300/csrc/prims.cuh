@@ -7,7 +7,6 @@
 #include "device.cuh"
 
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 namespace sigma {
@@ -291,6 +290,7 @@ struct RadixShared {
     u32 start[256];             // the digit's first place in the tile
     u32 wtot[kRadixWarps];
 };
+static_assert(sizeof(RadixShared) <= 48 * 1024, "more shared memory needs an attribute per device");
 
 // Ranks of a tile's pairs: pair k of a lane (place warp * 512 + k * 32 + lane, those from
 // n on left out) goes to place rank[k] of the tile ordered by digit. Thread d gets the
@@ -483,11 +483,6 @@ inline size_t radix_work_elems(size_t n) { return 1024 + 4 + 256 * radix_tiles(n
 inline bool radix_sort_any(u32* keys, u32* vals, u32* k2, u32* v2, size_t n, int bits, u64* work, u32* err,
                            cudaStream_t s, unsigned& launches) {
     if (n <= 1) return false;
-    static std::once_flag attr;
-    std::call_once(attr, [] {
-        cudaFuncSetAttribute(radix_pass_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RadixShared));
-        cudaFuncSetAttribute(radix_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RadixShared));
-    });
     const int passes = (bits + 7) / 8;
     if (n <= (size_t)kRadixTile) {
         launches++;

@@ -1159,6 +1159,7 @@ struct pf_sigma_ctx {
 #if SIGMA_CUDA
         if (npvs) {
             const int smem = SORT_WARPS * (int)sizeof(SortStage);
+            static_assert(SORT_WARPS * sizeof(SortStage) <= 48 * 1024, "more shared memory needs an attribute");
             rt.launches++;
             sort_lists_k<<<rt.grid((npvs + 15) / 16 * 32), SORT_WARPS * 32, smem, rt.stream>>>(a);
             ck(cudaGetLastError(), "launch");
@@ -2522,6 +2523,7 @@ pf_status pf_sigma_round(pf_sigma_ctx* ctx, pf_round_stats* stats) {
     c.whole.reset();
     c.ph_open = -1;
     c.ot_total_due = false;
+    c.slots = ReadSlots{};  // (a round that stopped may have left some)
     pf_status status = PF_OK;
     try {
         c.keep_at.reserve(c.rt, (size_t)c.nvars + 1);

@@ -105,3 +105,14 @@ def test_prop_gpu(cuda_lib, built, name, sweep_div):
 @pytest.mark.gpu
 def test_prop_batch_gpu(cuda_lib, built):
     _check_batch(cuda_lib)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("depth", [1, 2, 9, 40])
+def test_prop_loop_limit_gpu(cuda_lib, built, depth):
+    """The loop bound that a propagation level by level (the serial waves) just keeps."""
+    nv, lits, off = _pack(depth + 1, [[1]] + [[-i, i + 1] for i in range(1, depth)] + [[-depth, depth + 1]])
+    stats, _, _ = run_lib(built["emu"], nv, lits, off, Options(all=1, sweep_div=-1), level=1)
+    assert stats.status == 0 and stats.prop_waves >= depth
+    opts = Options(all=1, sweep_div=-1, loop_limit=int(stats.prop_waves))
+    assert run_lib(cuda_lib, nv, lits, off, opts, level=1)[0].status == 0
