@@ -293,10 +293,13 @@ class Simplifier:
     # ---- formula batches
     def awaken_batch(self, formulas) -> None:
         """Upload a batch: formulas is a sequence of (num_vars, lits, offsets) in each
-        formula's own numbering (each formula copied from its own arrays)."""
+        formula's own numbering (each formula read from its own arrays)."""
         nf = len(formulas)
         arrs = [(np.ascontiguousarray(l, dtype=np.uint32), np.ascontiguousarray(o, dtype=np.uint64))
                 for _, l, o in formulas]
+        # the device reads the arrays in place: a range past an array's end stops here
+        if any(o.size and int(o[-1]) > l.size for l, o in arrs):
+            raise SigmaError(PF_EINVAL, "offsets past the literals")
         nv = np.array([f[0] for f in formulas], dtype=np.uint32)
         nc = np.array([o.size - 1 for _, o in arrs], dtype=np.uint64)
         dummy = np.zeros(1, np.uint32)  # stands for an empty formula's literal array

@@ -7,7 +7,7 @@ import pytest
 
 from parafrost_gb300 import cnfgen, rounddump as rd
 from parafrost_gb300.options import Options
-from parafrost_gb300.sigma import Simplifier, lits_offsets_begin, pack_batch
+from parafrost_gb300.sigma import PF_EINVAL, SigmaError, Simplifier, lits_offsets_begin, pack_batch
 
 
 def _shifted(a, by):
@@ -56,3 +56,12 @@ def test_parts_emu(built, shift):
 @pytest.mark.parametrize("shift", [0, 4, 8, 2, 1])
 def test_parts_gpu(cuda_lib, shift):
     _check(cuda_lib, shift)
+
+
+def test_parts_past_the_literals_emu(built):
+    good = cnfgen.random_ksat(3, 4, 3, seed=1)
+    bad = (3, good[1][:-1].copy(), good[2])  # the last clause's last literal is missing
+    with Simplifier(Options(all=1), library=built["emu"]) as s:
+        with pytest.raises(SigmaError) as e:
+            s.awaken_batch([good, bad])
+        assert e.value.status == PF_EINVAL
