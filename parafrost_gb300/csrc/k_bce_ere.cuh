@@ -47,19 +47,20 @@ HD bool bce_blocked(const Ctx& c, u32 v, const Hdr& neg, const ListRef& poss) {
 // elected variable: the lanes take the negative clauses, each checking its own
 // against the whole positive list. A variable eliminated by VE in this phase is
 // skipped (PVs[i] == 0 in the reference).
+HD bool bce_skip(const BceArgs& a, u32 k) {
+    const Ctx& c = a.c;
+    const u32 v = a.pvs[k], p = V2L(v);
+    return c.vstate[v] || c.ot_size[p] > a.bce_max || c.ot_size[NEG(p)] > a.bce_max;
+}
 HD void bce_count_warp(const BceArgs& a, u32 k) {
     const Ctx& c = a.c;
     const u32 v = a.pvs[k];
     const u32 p = V2L(v), n = NEG(p);
-    const bool skip = c.vstate[v] || c.ot_size[p] > a.bce_max || c.ot_size[n] > a.bce_max;
-    u32 w = 0;
-    if (!skip) {
-        const ListRef poss = list_of(c, p), negs = list_of(c, n);
-        w = wsum(negs.n, [&](u32 i) {
-            const Hdr neg = c.hdr[negs.ids[i]];
-            return (h_original(neg.flags) && bce_blocked(c, v, neg, poss)) ? neg.size + 1 : 0u;
-        });
-    }
+    const ListRef poss = list_of(c, p), negs = list_of(c, n);
+    const u32 w = wsum(negs.n, [&](u32 i) {
+        const Hdr neg = c.hdr[negs.ids[i]];
+        return (h_original(neg.flags) && bce_blocked(c, v, neg, poss)) ? neg.size + 1 : 0u;
+    });
     wone([&] { a.nwit[k] = w; });
 }
 
@@ -74,7 +75,12 @@ __global__ void __launch_bounds__(256) bce_count_warp_k(BceArgs a, const u32* pe
         j0 = __shfl_sync(0xffffffffu, j0, 0);
         if (j0 >= npos) break;
         const u32 j1 = j0 + chunk < npos ? j0 + chunk : npos;
-        for (u32 j = j0; j < j1; j++) bce_count_warp(a, perm[j]);
+        // a skipped variable of the grab costs one lane's loads
+        const u32 kq = j0 + lane < j1 ? perm[j0 + lane] : 0u;
+        const bool skip = j0 + lane < j1 && bce_skip(a, kq);
+        if (skip) a.nwit[kq] = 0;
+        for (u32 m = __ballot_sync(kFull, j0 + lane < j1 && !skip); m; m &= m - 1u)
+            bce_count_warp(a, __shfl_sync(kFull, kq, __ffs(m) - 1));
         chunk = warp_chunk(npos - j1);
     }
 }

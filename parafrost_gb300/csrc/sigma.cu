@@ -98,7 +98,8 @@ struct FSubWarp {
     SubArgs a;
     HD void operator()(u32 k) const {
         u32 slot[SUB_SLOT];
-        sub_warp_pv(a, k, slot);
+        SubHead h;
+        if (sub_head(a, k, h)) sub_warp_pv(a, h, slot);
     }
 };
 struct FSubCommitSize { Ctx c; const u32* lits; u32* size; HD void operator()(u32 q) const { k_sub_commit_size(c, lits, size, q); } };
@@ -110,7 +111,13 @@ struct FSubCommitClear { Ctx c; const u32* lits; HD void operator()(u32 q) const
 struct FSubAssign { Ctx c; const U2* units; HD void operator()(u32 i) const { enqueue_unit(c, units[i].y); } };
 struct FBveWarp { BveArgs a; HD void operator()(u32 i) const { k_bve_warp(a, i); } };
 struct FBveWrite { BveArgs a; HD void operator()(u32 i) const { k_bve_write(a, i); } };
-struct FBceCountWarp { BceArgs a; HD void operator()(u32 i) const { bce_count_warp(a, i); } };
+struct FBceCountWarp {
+    BceArgs a;
+    HD void operator()(u32 i) const {
+        if (bce_skip(a, i)) a.nwit[i] = 0;
+        else bce_count_warp(a, i);
+    }
+};
 struct FBceWrite { BceArgs a; HD void operator()(u32 i) const { k_bce_write(a, i); } };
 struct FEre { EreArgs a; HD void operator()(u32 i) const { k_ere_pv(a, i); } };
 struct FEreCount { EreArgs a; const u32* perm; u64* cnt; HD void operator()(u32 q) const { k_ere_count(a, perm, cnt, q); } };
@@ -866,6 +873,9 @@ struct pf_sigma_ctx {
         return (u32)std::min<u64>(std::max<u64>(mean, 1), 0xFFFFFFFFull);
     }
     // Blocks of the per-variable warp kernels.
+    // More variables than warps at six blocks an SM (the per-variable kernels that wait on
+    // memory then run eight).
+    bool pv_many(u32 n) const { return n > (u32)rt.sms * 48u; }
     u32 pv_grid() const { return (u32)rt.sms * (opt.pv_blocks > 0 ? (u32)opt.pv_blocks : 8u); }
 
 #if SIGMA_CUDA
@@ -1212,7 +1222,8 @@ struct pf_sigma_ctx {
         if (!perm_n) return;
         ck(cudaMemsetAsync(counters.p + 11, 0, 4, rt.stream), "memset");
         rt.launches++;
-        sub_warp_k<<<pv_grid(), 256, 0, rt.stream>>>(a, pv_perm.p + perm_off, perm_n, counters.p + 11);
+        (pv_many(perm_n) ? sub_warp_k<8> : sub_warp_k<6>)<<<pv_grid(), 256, 0, rt.stream>>>(a, pv_perm.p + perm_off, perm_n,
+                                                                                          counters.p + 11);
         ck(cudaGetLastError(), "launch");
 #else
         pv_each(FSubWarp{a});
@@ -1488,8 +1499,8 @@ struct pf_sigma_ctx {
         if (perm_n) {
             ck(cudaMemsetAsync(counters.p + 11, 0, 4, rt.stream), "memset");
             rt.launches++;
-            bve_write_warp_k<<<pv_grid(), 256, 0, rt.stream>>>(a, pv_perm.p + perm_off, perm_n,
-                                                                       counters.p + 11);
+            (pv_many(perm_n) ? bve_write_warp_k<8> : bve_write_warp_k<6>)<<<pv_grid(), 256, 0, rt.stream>>>(
+                a, pv_perm.p + perm_off, perm_n, counters.p + 11);
             ck(cudaGetLastError(), "launch");
         }
 #else
