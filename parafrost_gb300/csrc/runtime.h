@@ -93,14 +93,15 @@ struct Runtime {
     size_t budget = 0;  // 0 = no limit
     unsigned launches = 0;
     unsigned syncs = 0;  // host waits for the device (synchronous reads, stream and event syncs)
-    // page-locked host memory that short reads go through: a copy to pageable memory is
-    // staged by the driver
+    // page-locked host memory that short reads go through (a copy to pageable memory is
+    // staged by the driver), and behind it the words that read_slots_k writes
     static constexpr size_t kPinBytes = 4096;
     void* pin = nullptr;
+    u64* pin_slots() const { return (u64*)((char*)pin + kPinBytes); }
 
     void init_pin() {
 #if SIGMA_CUDA
-        ck(cudaMallocHost(&pin, kPinBytes), "host alloc");
+        ck(cudaMallocHost(&pin, kPinBytes + 8 * sizeof(u64)), "host alloc");
 #endif
     }
     void init() {

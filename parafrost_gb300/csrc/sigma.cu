@@ -492,22 +492,33 @@ struct pf_sigma_ctx {
     }
     // All slots into hr. The error word rides along in slot 7 and is checked, the trail's
     // length in slot 6, and the last table's size where it has not been read yet.
+    // queue_slots writes them, take_slots_checked takes them once the host has waited for
+    // the stream.
     bool ot_total_due = false;
-    void read_slots_checked(u32 stage_err_mask = ~0u) {
+    void queue_slots() {
         word_to(counters.p + 1, 7);
         word_to(counters.p + 0, 6);
         if (ot_total_due) word_to(ot_off.p + D, 5);
 #if SIGMA_CUDA
         rt.launches++;
-        rt.syncs++;
-        read_slots_k<<<1, 32, 0, rt.stream>>>(slots, (u64*)rt.pin);
+        read_slots_k<<<1, 32, 0, rt.stream>>>(slots, rt.pin_slots());
         ck(cudaGetLastError(), "launch");
-        ck(cudaStreamSynchronize(rt.stream), "sync");
-        std::memcpy(hr, rt.pin, sizeof hr);
 #else
         for (int k = 0; k < 8; k++) hr[k] = read_slot(slots, k);
 #endif
         slots = ReadSlots{};
+    }
+    void read_slots_checked(u32 stage_err_mask = ~0u) {
+        queue_slots();
+#if SIGMA_CUDA
+        rt.sync();
+#endif
+        take_slots_checked(stage_err_mask);
+    }
+    void take_slots_checked(u32 stage_err_mask = ~0u) {
+#if SIGMA_CUDA
+        std::memcpy(hr, rt.pin_slots(), sizeof hr);
+#endif
         ntrail = (u32)hr[6];
         if (ot_total_due) alg_bytes += 4ull * (u32)hr[5];
         ot_total_due = false;
@@ -1513,8 +1524,8 @@ struct pf_sigma_ctx {
         nlits_used += add_lits;
         proof_clauses(first_new);
         nresolved += add_wit;
-        // the units and the error word are read with the next stage's values (BCE and the
-        // counts) unless stage dumps are being recorded
+        // the units and the error word are read with the next stage's values (BCE, and the
+        // counts where BCE is off) unless stage dumps are being recorded
         if (opt.dump_level) read_slots_checked();
         alg_bytes += 4ull * add_lits + 8ull * add_cls + 4ull * add_wit;
     }
@@ -2018,7 +2029,11 @@ struct pf_sigma_ctx {
 #else
         rt.each(FCountFormula{a}, ncls);
 #endif
+        // the trail's length and the error word with the counts (BVE's write step leaves
+        // both to the next read, as count_all's of a single formula)
+        queue_slots();
         std::vector<u64> h = fetch(f_count.p, 2 * (size_t)nf);
+        take_slots_checked();
         fc_cls.assign(h.begin(), h.begin() + nf);
         fc_lits.assign(h.begin() + nf, h.end());
         n_cls_after = n_lits_after = 0;
@@ -2279,11 +2294,13 @@ static pf_status upload_common(pf_sigma_ctx* ctx, uint32_t num_vars, const uint3
         c.nvars = num_vars;
         c.D = 2 * (num_vars + 1);
         c.nf = batch ? batch->nf : 0u;
-            c.fc_cls.clear();
+        c.fc_cls.clear();
         c.fc_lits.clear();
         c.ncls = (u32)num_clauses;
         c.nlits_used = L;
         c.ntrail = c.prop_head = 0;
+        c.slots = ReadSlots{};  // (a round that stopped may have left some)
+        c.ot_total_due = false;
         c.nresolved = 0;
         c.has_learnt = false;
         const size_t cap_cls = (size_t)num_clauses + num_clauses / 2 + 1024;
