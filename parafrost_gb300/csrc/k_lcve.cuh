@@ -589,19 +589,24 @@ DEV void mis_queue_flush(MisBlockQueue& q, const MisFront& f) {
 // wait: the neighbour that stopped the last try (0 or NONE: none known). Until it is
 // decided only its word and v's own are looked at: one load a try instead of a walk's
 // four dependent ones.
+// Other blocks decide both words at any time, and the lanes' loads need not be one access:
+// the group goes by what its first lane saw, so all of it takes the same branches (the
+// collectives below name every lane of the group).
 DEV bool mis_try(const LcveArgs& a, u32 v, u32 gm, u32 gbase, u32 sub, u32 L, u32& at, u32& wait, bool r0) {
-    const u32 wv = vload(&a.word[v]);  // the same word for the whole group
+    const u32 wv = vload(&a.word[v]);
     const bool known = wait && wait != NONE;
     const u32 ww = known ? vload(&a.word[wait]) : 0u;
-    if (mis_dec(wv) != MIS_UNDECIDED) return true;
+    const u32 seen = __shfl_sync(gm, mis_dec(wv) | mis_dec(ww) << 2, (int)gbase);
+    const u32 dv = seen & 3u, dw = seen >> 2;
+    if (dv != MIS_UNDECIDED) return true;
     if (known) {
-        if (mis_dec(ww) == MIS_UNDECIDED) return false;
-        if (mis_dec(ww) == MIS_IN) {  // a lower neighbour is in
+        if (dw == MIS_UNDECIDED) return false;
+        if (dw == MIS_IN) {  // a lower neighbour is in
             if (sub == 0) atomicOr(&a.word[v], mis_dec_bits(MIS_OUT));
             return true;
         }
     }
-    const u32 rv = mis_rank(wv);
+    const u32 rv = mis_rank(wv);  // (a word's rank does not change)
     const u32 p = V2L(v), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
     const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
     for (u32 b0 = at; b0 < n; b0 += L) {
