@@ -460,23 +460,16 @@ HD void mis_push_clause(const LcveArgs& a, u32 u, u32 ru, const MisCl& cl) {
     }
 }
 
-HD void mis_push_vertex(const LcveArgs& a, u32 u) {
-    const u32 ru = mis_rank(a.word[u]);
+#if !SIGMA_CUDA
+// Serial rounds of the emulation build: what went in marks its neighbours, then the
+// undecided vertices walk. (A list that has shrunk ends before the next one's start, so
+// an empty positive list's first clause is the negative one's.)
+HD void k_mis_push(const LcveArgs& a, const u32* in, u32 idx) {
+    const u32 u = in[idx], ru = mis_rank(a.word[u]);
     const u32 p = V2L(u), np = a.c.ot_size[p], n = np + a.c.ot_size[p + 1];
     const u32 op = a.c.ot_off[p], on = a.c.ot_off[p + 1] - np;
-    if (!n) return;
-    MisCl cl = mis_cl(a, ldro_hint(&a.c.ot_refs[op], a.pf), false);
-    for (u32 t = 0; t < n; t++) {
-        MisCl nx = cl;
-        if (t + 1 < n) nx = mis_cl(a, ldro_hint(&a.c.ot_refs[t + 1 < np ? op + t + 1 : on + t + 1], a.pf), false);
-        mis_push_clause(a, u, ru, cl);
-        cl = nx;
-    }
+    for (u32 t = 0; t < n; t++) mis_push_clause(a, u, ru, mis_cl(a, a.c.ot_refs[t < np ? op + t : on + t], false));
 }
-
-#if !SIGMA_CUDA
-// Serial rounds of the emulation build: the same phases over the same lists.
-HD void k_mis_push(const LcveArgs& a, const u32* in, u32 idx) { mis_push_vertex(a, in[idx]); }
 HD void k_mis_pull(const LcveArgs& a, const u32* in, const MisFront& und, const MisFront& ins, bool r0, u32 idx) {
     const u32 v = in[idx];
     const u32 wv = a.word[v];
