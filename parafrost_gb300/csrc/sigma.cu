@@ -777,6 +777,10 @@ struct pf_sigma_ctx {
     // with 16.4M 1.28 and 1.71, 33M 2.74 and 3.09, 66M 6.4 and 6.3.
     static constexpr u64 kOtbMinBytes = 7ull << 24;
     DBuf<u32> otb_count, otb_base, otb_cursor;
+    // Shared memory above 48 KB is asked for by every context: the attribute belongs to a
+    // kernel on a device, and a flag for the whole process would speak for other devices and
+    // for other copies of this library.
+    bool otb_smem_set = false, bve_smem_set = false;
     DBuf<u32> otb_cid;
     DBuf<unsigned short> otb_slot;
     bool otb_plan(u32& shift, u32& nb) const {
@@ -806,15 +810,14 @@ struct pf_sigma_ctx {
             (u32)std::min<u64>(std::max<u64>(std::min(by_stage, by_grid), 32), OTB_MAX_TILE) & ~31u;
         OtbArgs a{view(), shift, nb, otb_count.p, otb_cursor.p, otb_base.p, otb_cid.p, otb_slot.p, fill_tile};
         const u32 fill_smem = OTB_FILL_CAP * 6 + 2 * nb * 4;
-        static bool attr_set = false;
-        if (!attr_set) {
+        if (!otb_smem_set) {
             ck(cudaFuncSetAttribute(ot_bucket_lists_k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)((1u << OTB_MAX_SHIFT) * 4)),
                "smem attr");
             ck(cudaFuncSetAttribute(ot_bucket_fill_k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)(OTB_FILL_CAP * 6 + 2 * OTB_MAX_BUCKETS * 4)),
                "smem attr");
-            attr_set = true;
+            otb_smem_set = true;
         }
         const u32 grid = (u32)rt.sms * 8u;
         if (ncls) {
@@ -1469,10 +1472,9 @@ struct pf_sigma_ctx {
 #if SIGMA_CUDA
         {
             const int smem = kBveWarpThreads / 32 * (int)WPV_WORDS * 4;
-            static bool attr_set = false;
-            if (!attr_set) {
+            if (!bve_smem_set) {
                 ck(cudaFuncSetAttribute(bve_warp_k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attr");
-                attr_set = true;
+                bve_smem_set = true;
             }
             ck(cudaMemsetAsync(counters.p + 11, 0, 4, rt.stream), "memset");
             rt.launches++;
