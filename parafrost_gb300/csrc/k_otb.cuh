@@ -34,9 +34,12 @@ namespace sigma {
 #if SIGMA_CUDA
 
 constexpr u32 OTB_FILL_CAP = 14336;  // occurrences of a pass-1 tile ordered in shared memory
-                                     // (84 KB: two blocks per SM)
+                                     // (84 KB)
 constexpr u32 OTB_MAX_TILE = 1u << 16;  // clauses of a pass-1 tile
 constexpr u32 OTB_MAX_BUCKETS = 4096;
+constexpr u32 OTB_FILL_BUCKETS = 3680;  // most buckets with which two blocks of pass 1 fit an SM
+static_assert(2 * (OTB_FILL_CAP * 6 + 8 * (OTB_FILL_BUCKETS + 1) + 128 + 1024) <= 228 * 1024,
+              "stage, counters, static shared memory and the 1 KB a block reserves, twice");
 constexpr u32 OTB_MAX_SHIFT = 15;   // 32,768 slots: 128 KiB of shared counters in pass 2
 constexpr u32 OTB_LIST_THREADS = 1024;  // one block a bucket, 32 warps to keep its loads in flight
 constexpr unsigned OTB_FULL = 0xffffffffu;

@@ -785,10 +785,12 @@ struct pf_sigma_ctx {
     DBuf<unsigned short> otb_slot;
     bool otb_plan(u32& shift, u32& nb) const {
         if (opt.ot_buckets < 0 || (opt.ot_buckets == 0 && 4ull * (nlits_used + D) < kOtbMinBytes)) return false;
-        // some 2,000 buckets, 4,000 for tables that are much larger than L2 (tables of a
+        // some 2,000 buckets, more for tables that are much larger than L2 (tables of a
         // round at 512, 1,024, 2,048 and 4,096: 28M occurrences 1.29, 1.24, 1.23 and 1.61 ms,
-        // 50M of a batch 5.30, 4.57, 4.29 and 5.12, 280M 13.5, 13.5, 13.5 and 13.1)
-        const u64 most = nlits_used >= (1ull << 27) ? 4096 : 2048;
+        // 50M of a batch 5.30, 4.57, 4.29 and 5.12, 280M 13.5, 13.5, 13.5 and 13.1), up to what
+        // leaves room for two blocks of the fill on an SM (168M occurrences over 32M literal
+        // slots: 3,907 buckets and one block 9.5 ms, 1,954 and two 7.8)
+        const u64 most = nlits_used >= (1ull << 27) ? OTB_FILL_BUCKETS : 2048;
         u32 s = 8;
         while (s < OTB_MAX_SHIFT && ((u64)D >> s) > most) s++;
         shift = s;
