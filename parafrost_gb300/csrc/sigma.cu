@@ -1232,10 +1232,12 @@ struct pf_sigma_ctx {
         sub_units_possible = hr[2] != 0;
     }
 
-    // One SUB pass over the elected variables (warp per variable).
+    // One SUB pass over the elected variables (warp per variable); the kernel's clock runs
+    // over all passes of a round.
     void sub_pass(const SubArgs& a) {
-#if SIGMA_CUDA
         if (!perm_n) return;
+        kclock[K_SUB].start(rt);
+#if SIGMA_CUDA
         ck(cudaMemsetAsync(counters.p + 11, 0, 4, rt.stream), "memset");
         rt.launches++;
         (pv_many(perm_n) ? sub_warp_k<8> : sub_warp_k<6>)<<<pv_grid(), 256, 0, rt.stream>>>(a, pv_perm.p + perm_off, perm_n,
@@ -1244,6 +1246,7 @@ struct pf_sigma_ctx {
 #else
         pv_each(FSubWarp{a});
 #endif
+        kclock[K_SUB].stop(rt);
     }
 
     // SUB (elimination.cpp:110-129).
@@ -1263,9 +1266,7 @@ struct pf_sigma_ctx {
         a.run = nullptr;
         kbytes[K_SUB] += phase_ws;
         if (!sub_units_possible) {
-            kclock[K_SUB].start(rt);
             sub_pass(a);
-            kclock[K_SUB].stop(rt);
             // the exact pass derives no unit; its error word is read with the next
             // stage's values (the VE preparation and the counts only read the store)
             // unless stage dumps are being recorded
@@ -1355,9 +1356,7 @@ struct pf_sigma_ctx {
         a.cap_units = (u32)sub_units.n;
         a.run = fx_prod8.p;
         write_u32(counters.p + 4, 0);
-        kclock[K_SUB].start(rt);
         sub_pass(a);
-        kclock[K_SUB].stop(rt);
         check();
         u32 nu = read_u32(counters.p + 4);
         // fix-point among the producers: a producer re-runs when the set of earlier
