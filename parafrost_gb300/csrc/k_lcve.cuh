@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256) mis_init_k(LcveArgs a, MisFront und, u32 
 constexpr u32 MIS_CHUNK = 4;
 
 // A clause as the election reads it: one 16-byte record holding its first three
-// literals and its size and deleted bit (built once per election by k_mis_rec), so
+// literals and its size and deleted bit (built once per election), so
 // clauses of up to three literals cost one load; longer ones read the rest of
 // their literals from the store.
 // In the first round no vertex is out yet, so a clause stops a walk of v exactly when
@@ -243,6 +243,7 @@ HD const u32* mis_long_lits(const LcveArgs& a, const MisCl& cl) {
 // The record of clause i, its least graph rank, and the graph's working set: every graph
 // vertex's list entry (4 bytes) and, for a live clause, its header and literals
 // (8 + 4*len) once per graph vertex in it. Runs after the graph is known.
+#if !SIGMA_CUDA
 HD void k_mis_rec(const LcveArgs& a, Q4* rec, u32 i) {
     const Ctx& c = a.c;
     const Hdr h = c.hdr[i];
@@ -262,9 +263,8 @@ HD void k_mis_rec(const LcveArgs& a, Q4* rec, u32 i) {
     a.cmin[i] = h_deleted(h.flags) ? MIS_NO_RANK : m;
     spread_sum_add64(a.ws_bytes, (u64)ng * (4ull + (h_deleted(h.flags) ? 0ull : 8ull + 4ull * h.size)));
 }
-
-#if SIGMA_CUDA
-// k_mis_rec for 32 clauses per warp: lane i writes the record of clause id0 + i
+#else
+// The same for 32 clauses per warp: lane i writes the record of clause id0 + i
 // (coalesced 16-byte stores), and the graph working set is summed over the warp's
 // literals with consecutive lanes on consecutive literals (coalesced reads), each
 // literal of a graph vertex adding 4 bytes and, in a live clause, the clause's

@@ -27,57 +27,39 @@ struct PropArgs {
     u32 head;        // first pending trail index of this wave
     u32 stamp;       // wave stamp (not used before; the launch of all waves takes one per wave)
     u32* cl_stamp;   // per clause: last wave that collected it
+#if !SIGMA_CUDA
     u32* work;       // collected clause ids
-    u32* nwork;      // device counter
+    u32* nwork;      // their count
     u32 cap_work;
+#endif
 };
 
-// Loads of data that other blocks of the same launch may have written (the
-// persistent wave kernel): read at L2, past this SM's L1.
-template <bool Fresh, class T>
-HD T ldw(const T* p) {
-#if defined(__CUDA_ARCH__)
-    if (Fresh) return __ldcg(p);
-#endif
-    return *p;
-}
-template <bool Fresh>
-HD Hdr ldw_hdr(const Hdr* p) {
-#if defined(__CUDA_ARCH__)
-    if (Fresh) {
-        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p));
-        Hdr h;
-        h.start = v.x;
-        h.size = v.y;
-        h.sig = v.z;
-        h.flags = v.w;
-        return h;
-    }
-#endif
-    return *p;
-}
+constexpr u32 PROP_SHORT = 4;  // literals of a clause loaded together
 
+#if !SIGMA_CUDA
+// The waves of the emulation build, one item after another. They share the fixpoint with
+// the GPU's waves, not their walks, chases, list parts and strip: those run on a GPU only.
+//
 // Wave A: one item per pending literal.
-template <bool Fresh>
-HD void prop_lists(const PropArgs& a, u32 k) {
+HD void k_prop_lists(const PropArgs& a, u32 k) {
     const Ctx& c = a.c;
-    const u32 t = ldw<Fresh>(&c.trail[a.head + k]);
+    const u32 t = c.trail[a.head + k];
     const u32 f = FLIP(t);
     // collect ot[-t]
-    const u32 fo = c.ot_off[f], fs = ldw<Fresh>(&c.ot_size[f]);
+    const u32 fo = c.ot_off[f], fs = c.ot_size[f];
     for (u32 i = 0; i < fs; i++) {
         const u32 r = c.ot_refs[fo + i];
-        const bool take = !h_deleted(ldw<Fresh>(&c.hdr[r].flags)) && atom_exch(&a.cl_stamp[r], a.stamp) != a.stamp;
+        const bool take = !h_deleted(c.hdr[r].flags) && atom_exch(&a.cl_stamp[r], a.stamp) != a.stamp;
         const u32 pos = warp_append(a.nwork, take);  // one reservation per group of lanes
         if (!take) continue;
         if (pos < a.cap_work) a.work[pos] = r;
         else set_err(c, ERR_CAP_SCRATCH);
     }
     // toblivion(ot[t])
-    const u32 to = c.ot_off[t], ts = ldw<Fresh>(&c.ot_size[t]);
+    const u32 to = c.ot_off[t], ts = c.ot_size[t];
     for (u32 i = 0; i < ts; i++) {
         const u32 r = c.ot_refs[to + i];
-        c.hdr[r].flags = (ldw<Fresh>(&c.hdr[r].flags) & ~3u) | ST_DELETED;
+        c.hdr[r].flags = (c.hdr[r].flags & ~3u) | ST_DELETED;
         touch(c, r);
     }
     c.ot_size[t] = 0;
@@ -85,22 +67,20 @@ HD void prop_lists(const PropArgs& a, u32 k) {
 }
 
 // Wave B: one item per collected clause.
-constexpr u32 PROP_SHORT = 4;
-template <bool Fresh>
-HD void prop_clause(const PropArgs& a, u32 k) {
+HD void k_prop_clause(const PropArgs& a, u32 k) {
     const Ctx& c = a.c;
-    const u32 r = ldw<Fresh>(&a.work[k]);
-    Hdr h = ldw_hdr<Fresh>(&c.hdr[r]);
+    const u32 r = a.work[k];
+    Hdr h = c.hdr[r];
     if (h_deleted(h.flags)) return;
     u32* l = c.lits + h.start;
-    const u32 v0 = ABS(ldw<Fresh>(&l[0]));  // names the formula if the clause empties
+    const u32 v0 = ABS(l[0]);  // names the formula if the clause empties
     u32 n = 0, sig = 0;
     if (h.size <= PROP_SHORT) {
         // short clause: all literals and their values loaded together
         u32 L[PROP_SHORT];
         int val[PROP_SHORT];
 #pragma unroll
-        for (u32 j = 0; j < PROP_SHORT; j++) L[j] = j < h.size ? ldw<Fresh>(&l[j]) : 0u;
+        for (u32 j = 0; j < PROP_SHORT; j++) L[j] = j < h.size ? l[j] : 0u;
 #pragma unroll
         for (u32 j = 0; j < PROP_SHORT; j++) val[j] = j < h.size ? lit_value(c, L[j]) : 0;
         bool sat = false;
@@ -121,14 +101,14 @@ HD void prop_clause(const PropArgs& a, u32 k) {
     } else {
         // satisfied?
         for (u32 i = 0; i < h.size; i++) {
-            if (lit_value(c, ldw<Fresh>(&l[i])) == 1) {
+            if (lit_value(c, l[i]) == 1) {
                 c.hdr[r].flags = (h.flags & ~3u) | ST_DELETED;
                 touch(c, r);
                 return;
             }
         }
         for (u32 i = 0; i < h.size; i++) {
-            const u32 lit = ldw<Fresh>(&l[i]);
+            const u32 lit = l[i];
             if (lit_value(c, lit) == 0) continue;
             l[n++] = lit;
             sig |= MAPHASH(lit);
@@ -150,9 +130,62 @@ HD void prop_clause(const PropArgs& a, u32 k) {
     if (n == 1) claim_unit(c, l[0]);
 }
 
-HD void k_prop_lists(const PropArgs& a, u32 k) { prop_lists<false>(a, k); }
-
-#if SIGMA_CUDA
+// Sweep wave: when the pending literals' lists cover a large part of the store (a
+// propagation cascade), every clause of the store is checked against the current
+// assignment instead, in store order (streaming reads, no list walk, no collection):
+// a clause with a true literal is deleted, one with false literals loses them (a
+// unit is claimed, an empty clause is a conflict); a clause without an assigned
+// literal is left alone. Literals assigned during the sweep are pending for the next
+// wave, so the fixpoint is the one the list waves reach.
+HD void k_prop_sweep(const PropArgs& a, u32 r) {
+    const Ctx& c = a.c;
+    Hdr h = c.hdr[r];
+    if (h_deleted(h.flags)) return;
+    u32* l = c.lits + h.start;
+    u32 nfalse = 0;
+    for (u32 i = 0; i < h.size; i++) {
+        const int v = lit_value(c, l[i]);
+        if (v == 1) {
+            c.hdr[r].flags = (h.flags & ~3u) | ST_DELETED;
+            touch(c, r);
+            return;
+        }
+        nfalse += v == 0;
+    }
+    if (!nfalse) return;
+    const u32 v0 = ABS(l[0]);
+    u32 n = 0, sig = 0;
+    for (u32 i = 0; i < h.size; i++) {
+        const u32 lit = l[i];
+        if (lit_value(c, lit) == 0) continue;
+        l[n++] = lit;
+        sig |= MAPHASH(lit);
+    }
+    h.size = n;
+    h.sig = sig;
+    c.hdr[r] = h;
+    touch(c, r);
+    if (n == 0) {
+        set_unsat(c, v0);
+        if (c.var_fid) {
+            c.hdr[r].flags = (h.flags & ~3u) | ST_DELETED;
+            touch(c, r);
+        }
+        return;
+    }
+    if (n == 1) claim_unit(c, l[0]);
+}
+// The lists of a swept wave's literals end empty, as the list waves leave them.
+HD void k_prop_sweep_lists(const PropArgs& a, u32 k) {
+    const u32 t = a.c.trail[a.head + k];
+    a.c.ot_size[t] = 0;
+    a.c.ot_size[FLIP(t)] = 0;
+}
+// Sweep rather than walk: the pending literals' lists (estimated from the mean list
+// length) exceed a fraction of the store; scale = mean list length x the divisor of
+// that fraction (0: never sweep).
+HD bool prop_use_sweep(u32 pending, u32 scale, u32 ncls) { return scale && (u64)pending * scale > (u64)ncls; }
+#else
 // Clause r, which holds a literal that has become false, judged against the current
 // assignment (read at L2: other warps assign meanwhile) without being changed, except
 // that a clause with a true literal is deleted. Two unassigned literals end the look (a
@@ -370,77 +403,22 @@ DEV void prop_chase(const Ctx& c, const PropOut& o, PropWarp& s, u32 t, u32 s0, 
         __syncwarp();
     }
 }
-#endif
-HD void k_prop_clause(const PropArgs& a, u32 k) { prop_clause<false>(a, k); }
 
-// Sweep wave: when the pending literals' lists cover a large part of the store (a
-// propagation cascade), every clause of the store is checked against the current
-// assignment instead, in store order (streaming reads, no list walk, no collection):
-// a clause with a true literal is deleted, one with false literals loses them (a
-// unit is claimed, an empty clause is a conflict); a clause without an assigned
-// literal is left alone. Literals assigned during the sweep are pending for the next
-// wave, so the fixpoint is the one the list waves reach.
-template <bool Fresh>
-HD void prop_sweep_clause(const PropArgs& a, u32 r) {
-    const Ctx& c = a.c;
-    Hdr h = ldw_hdr<Fresh>(&c.hdr[r]);
-    if (h_deleted(h.flags)) return;
-    u32* l = c.lits + h.start;
-    u32 nfalse = 0;
-    for (u32 i = 0; i < h.size; i++) {
-        const int v = lit_value(c, ldw<Fresh>(&l[i]));
-        if (v == 1) {
-            c.hdr[r].flags = (h.flags & ~3u) | ST_DELETED;
-            touch(c, r);
-            return;
-        }
-        nfalse += v == 0;
-    }
-    if (!nfalse) return;
-    const u32 v0 = ABS(ldw<Fresh>(&l[0]));
-    u32 n = 0, sig = 0;
-    for (u32 i = 0; i < h.size; i++) {
-        const u32 lit = ldw<Fresh>(&l[i]);
-        if (lit_value(c, lit) == 0) continue;
-        l[n++] = lit;
-        sig |= MAPHASH(lit);
-    }
-    h.size = n;
-    h.sig = sig;
-    c.hdr[r] = h;
-    touch(c, r);
-    if (n == 0) {
-        set_unsat(c, v0);
-        if (c.var_fid) {
-            c.hdr[r].flags = (h.flags & ~3u) | ST_DELETED;
-            touch(c, r);
-        }
-        return;
-    }
-    if (n == 1) claim_unit(c, l[0]);
-}
-HD void k_prop_sweep(const PropArgs& a, u32 r) { prop_sweep_clause<false>(a, r); }
-// The lists of a swept wave's literals end empty, as the list waves leave them.
-HD void k_prop_sweep_lists(const PropArgs& a, u32 k) {
-    const u32 t = a.c.trail[a.head + k];
-    a.c.ot_size[t] = 0;
-    a.c.ot_size[FLIP(t)] = 0;
-}
-// Sweep rather than walk: the pending literals' lists (estimated from the mean list
-// length) exceed a fraction of the store; scale = mean list length x the divisor of
-// that fraction (0: never sweep).
-HD bool prop_use_sweep(u32 pending, u32 scale, u32 ncls) { return scale && (u64)pending * scale > (u64)ncls; }
-
-#if SIGMA_CUDA
 // Header of clause r as another block may have left it; of no clause: deleted.
 DEV Hdr prop_hdr(const Ctx& c, u32 r, bool has) {
     Hdr h;
     h.start = h.size = h.sig = 0;
     h.flags = ST_DELETED;
-    if (has) h = ldw_hdr<true>(&c.hdr[r]);
+    if (has) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(&c.hdr[r]));
+        h.start = v.x;
+        h.size = v.y;
+        h.sig = v.z;
+        h.flags = v.w;
+    }
     return h;
 }
-// prop_clause (Always) or prop_sweep_clause (not Always) for up to 32 clauses by one
+// k_prop_clause (Always) or k_prop_sweep (not Always) for up to 32 clauses by one
 // warp: lane i holds the header of clause r; the live clauses' literals are then read and valued by consecutive lanes, 32 literals of the
 // warp's clauses per step, and each literal's value is read once. Every literal that
 // is not false moves down to its place among its clause's kept literals (it is
@@ -485,7 +463,7 @@ DEV u32 prop_warp_clauses(const PropArgs& a, u32* sm, u32 r, Hdr h) {
         const u32 st = __shfl_sync(0xffffffffu, h.start, k), ex = __shfl_sync(0xffffffffu, excl, k);
         const u32 kc = __shfl_sync(0xffffffffu, kept, k);  // the clause's literals kept in earlier steps
         const bool in = j < total;
-        const u32 lit = in ? ldw<true>(&c.lits[st + (j - ex)]) : 0u;
+        const u32 lit = in ? __ldcg(&c.lits[st + (j - ex)]) : 0u;
         const int val = in ? lit_value(c, lit) : VAL_UNDEF;
         const bool keep = in && val != 0;
         const u32 bt = __ballot_sync(0xffffffffu, in && val == 1), bf = __ballot_sync(0xffffffffu, in && val == 0);

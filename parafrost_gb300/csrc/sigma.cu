@@ -40,10 +40,12 @@ struct FHist { Ctx c; HD void operator()(u32 i) const { k_hist_clause(c, i); } }
 struct FScatter { Ctx c; HD void operator()(u32 i) const { k_scatter_clause(c, i); } };
 struct FOccursCl { Ctx c; HD void operator()(u32 i) const { k_occurs_clause(c, i); } };
 struct FCount { CountArgs a; HD void operator()(u32 i) const { k_count_clause(a, i); } };
+#if !SIGMA_CUDA
 struct FPropLists { PropArgs a; HD void operator()(u32 i) const { k_prop_lists(a, i); } };
 struct FPropClause { PropArgs a; HD void operator()(u32 i) const { k_prop_clause(a, i); } };
 struct FPropSweep { PropArgs a; HD void operator()(u32 i) const { k_prop_sweep(a, i); } };
 struct FPropSweepLists { PropArgs a; HD void operator()(u32 i) const { k_prop_sweep_lists(a, i); } };
+#endif
 struct FReduce { Ctx c; HD void operator()(u32 i) const { k_reduce_list(c, i); } };
 struct FRank { LcveArgs a; HD void operator()(u32 i) const { k_rank(a, i); } };
 #if !SIGMA_CUDA
@@ -945,8 +947,6 @@ struct pf_sigma_ctx {
             a.head = prop_head;
             a.stamp = wave_stamp + 1;
             a.cl_stamp = cl_stamp.p;
-            a.work = a.nwork = nullptr;  // (the serial waves' collected clauses)
-            a.cap_work = 0;
             // parts of long lists: a literal's lists are cut once, so all waves together
             // make at most one part per PROP_PART occurrences of the table
             const size_t nparts = (size_t)(nlits_used / PROP_PART) + 1024;
@@ -965,7 +965,7 @@ struct pf_sigma_ctx {
             w.sweep_scale = sweep_scale();
             w.sweep_div = sweep_div();
             if (trace_on) {
-                prop_trace.reserve(rt, 5 * kPropTraceWaves);
+                prop_trace.reserve(rt, 3 * kPropTraceWaves);
                 w.trace = prop_trace.p;
                 w.trace_cap = kPropTraceWaves - 1;
             }
@@ -1112,7 +1112,7 @@ struct pf_sigma_ctx {
         w.trace = nullptr;
         w.trace_cap = 0;
         if (trace_on) {
-            prop_trace.reserve(rt, 5 * kPropTraceWaves);
+            prop_trace.reserve(rt, 3 * kPropTraceWaves);
             w.trace = prop_trace.p;
             w.trace_cap = kPropTraceWaves;
         }
