@@ -88,7 +88,7 @@ typedef struct {
     double ms_stage[12];      /* ot, prop, lcve, sort, sub, ve, bce, ere, gc, count, upload, download */
     uint64_t algorithmic_bytes; /* bytes the round's kernels must move (HBM roofline numerator) */
     uint32_t kernel_launches;   /* kernels launched by the round */
-    uint32_t mis_rounds;        /* push/pull rounds of the independent-set elections */
+    uint32_t mis_rounds;        /* rounds of the independent-set elections */
     uint32_t prop_waves;        /* waves of the in-round unit propagations */
     uint32_t host_syncs;        /* times the host waited for the device during the round */
     /* The hottest kernels, timed with CUDA events on the context stream:

@@ -773,10 +773,13 @@ struct pf_sigma_ctx {
     // slots, at most OTB_MAX_BUCKETS of them (so up to 134M literal slots). Used when the
     // table and its counters (4 bytes an occurrence and a slot) outgrow 7/8 of the L2
     // cache, where the atomic histogram and scatter turn into random device-memory
-    // traffic. Tables of a round, atomics and buckets: 3-SAT with 12.6M occurrences 1.10
-    // and 1.05 ms, with 37.8M 5.6 and 2.9; community formulas with 21M 1.10 and 1.03, 28M
-    // 1.64 and 1.30, 56M 4.7 and 2.4; AIGs, whose clauses name neighbouring variables,
-    // with 16.4M 1.28 and 1.71, 33M 2.74 and 3.09, 66M 6.4 and 6.3.
+    // traffic. Tables of a round, atomics and buckets: mixed k-SAT with 19M occurrences
+    // 1.69 and 1.47 ms, 28M 3.15 and 2.11, 35M 4.37 and 2.63; community formulas with 19M
+    // 1.02 and 0.94, 28M 1.60 and 1.24, 35M 2.19 and 1.54. AIGs, whose clauses name
+    // neighbouring variables, keep most of their atomics in L2 up to larger tables: 20M
+    // 1.59 and 1.89, 35M 2.96 and 3.10, 49M 4.39 and 4.31. How far apart a formula's
+    // variables lie is not known before a pass over it, so the line goes by size: it costs
+    // the AIGs just above it 0.14 ms of a 27 ms round, and saves the others 0.4 to 1.7 ms.
     static constexpr u64 kOtbMinBytes = 7ull << 24;
     DBuf<u32> otb_count, otb_base, otb_cursor;
     // Shared memory above 48 KB is asked for by every context: the attribute belongs to a
